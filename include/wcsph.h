@@ -369,10 +369,8 @@ int32_t wcsph_sim_kernels_per_step(wcsph_sim* sim);
  * 2 and 4 sum in one order, 1 and 3 in another; 5 and 6 round P/rho^2
  * differently: results agree to FP32 rounding), out[2] log2 particle bucket
  * it was tuned for (-1:
- * defaults, not tuned), out[3] shape of the list build's scan (0-2 as out[0];
- * 3, 4: 4 or 8 warps per block with 256-candidate tiles; 5, 6: one lane per
- * particle walking a 512- or 256-candidate tile, 4 or 8 warps per block; all
- * build the same lists). */
+ * defaults, not tuned), out[3] shape of the list build's scan (0, 3, 5: 4
+ * warps per block, 1: 2, 2, 4, 6: 8; all build the same lists). */
 int wcsph_sim_tuning(wcsph_sim* sim, int32_t* out4);
 /* Neighbour-list counters (list_interval > 0): out[0] list builds, out[1]
  * steps that read the lists, out[2] builds whose lists overflowed (the next

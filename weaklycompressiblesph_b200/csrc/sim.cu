@@ -21,6 +21,7 @@
 #include "sim_kernels.cuh"
 #include "sim_aux.cuh"
 #include "sim_tiled.cuh"
+#include "sim_scan.cuh"
 #include "sim_slab.cuh"
 #include "sim_list.cuh"
 
@@ -284,8 +285,8 @@ static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, 
       k_hydro_plain<true><<<nblk(n), kBlock, 0, S.s>>>(a);
     } else if (build_lists) {  // the scan writes the lists, the list pass sums them
       const bool h16 = S.opt.precision == WCSPH_PREC_HALF2;
-      if (int rc = h16 ? launch_hydro_tiled<true, true>(a, n, S.s, S.build_shape)
-                       : launch_hydro_tiled<false, true>(a, n, S.s, S.build_shape))
+      if (int rc = h16 ? launch_list_scan<true>(a, n, S.s, S.build_shape)
+                       : launch_list_scan<false>(a, n, S.s, S.build_shape))
         return rc;
       if (ev && S.scan_ev) WCSPH_CUDA(cudaEventRecord(S.scan_ev, S.s));
       if (density) {
@@ -300,10 +301,8 @@ static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, 
                        : launch_hydro_list<false>(a, n, S.s, S.list_shape))
         return rc;
       ++L;
-    } else if (S.opt.precision == WCSPH_PREC_TILED) {
-      if (int rc = launch_hydro_tiled<false>(a, n, S.s, S.tile_shape)) return rc;
     } else {
-      if (int rc = launch_hydro_tiled<true>(a, n, S.s, S.tile_shape)) return rc;
+      if (int rc = launch_hydro_tiled(a, n, S.s, S.tile_shape)) return rc;
     }
     ++L;
     if (ev) WCSPH_CUDA(cudaEventRecord(ev[3], S.s));
@@ -445,9 +444,7 @@ static int autotune(SimImpl& S) {
   float best = 1e30f, ms = 0.f;
   int best_shape = 0;
   for (int v = 0; v < kTileShapes; ++v) {
-    int rc = time_launches(S, 3, [&]() {
-      return h16 ? launch_hydro_tiled<true>(a, n, S.s, v) : launch_hydro_tiled<false>(a, n, S.s, v);
-    }, &ms);
+    int rc = time_launches(S, 3, [&]() { return launch_hydro_tiled(a, n, S.s, v); }, &ms);
     if (rc) return rc;
     if (ms < best) best = ms, best_shape = v;
   }
@@ -479,9 +476,9 @@ static int autotune(SimImpl& S) {
     c.x0 = S.x0;
     float best_build = 1e30f;
     int best_build_shape = fixed_build > 0 ? fixed_build - 1 : 0;
-    for (int v = 0; v < kBuildShapes && fixed_build == 0; ++v) {
+    for (int v = 0; v < kBuildShapesTimed && fixed_build == 0; ++v) {
       int rc = time_launches(S, 3, [&]() {
-        return h16 ? launch_hydro_tiled<true, true>(c, n, S.s, v) : launch_hydro_tiled<false, true>(c, n, S.s, v);
+        return h16 ? launch_list_scan<true>(c, n, S.s, v) : launch_list_scan<false>(c, n, S.s, v);
       }, &ms);
       if (rc) return rc;
       if (ms < best_build) best_build = ms, best_build_shape = v;

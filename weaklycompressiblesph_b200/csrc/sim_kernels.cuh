@@ -345,7 +345,8 @@ __global__ void k_permute(StepArgs a) {
   // list build: the positions the lists refer to (kept by an instance that
   // keeps its lists in a partial build)
   const bool keep = a.inst_keep && a.list_flags[kLfPartial] != 0u && a.inst_keep[inst];
-  if (a.x0 && !keep) a.x0[p] = make_float4(x.x, x.y, x.z, 0.f);
+  if (a.x0 && !keep)  // w: the cell's low bits, a nibble per axis (cell_nibbles)
+    a.x0[p] = make_float4(x.x, x.y, x.z, __uint_as_float((cx & 3u) | ((cy & 3u) << 4) | ((cz & 3u) << 8)));
   if (f & kDeadBit) {  // removed during a partial build: in place until the next full build, far from all
     a.jr[p].a = make_float4(1.0e30f, 1.0e30f, 1.0e30f, 0.f);
     a.jr[p].b = make_float4(0.f, 0.f, 0.f, 1.f);

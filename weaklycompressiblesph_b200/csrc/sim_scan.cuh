@@ -1,0 +1,327 @@
+// Neighbour-list build: the scan that writes every particle's list row.
+//
+// One warp per non-empty cell, up to 32 of its particles at a time (lane l
+// holds particle l of the batch):
+//   1. The 27 neighbour cells are taken in the order of the cell search
+//      (for_each_neighbor).  Of three cells along x two are neighbours in the
+//      Morton order too, so that their particles are one run of slots: 18 runs
+//      are read instead of 27 ranges, with full 32-lane loads.
+//   2. A candidate is staged into the warp's shared-memory tile (SoA: x, y, z
+//      shifted by the periodic image, and its list entry) only when it lies
+//      within the list radius of the bounding box of the batch: about half
+//      of the 27 cells' particles do (729 -> 370 on a lattice with cells of
+//      2.3 h).
+//   3. Every lane tests 32 staged candidates at a time against its own
+//      particle (shared-memory broadcasts, packed f32x2 distances).  The sign
+//      of r^2 - R^2 is shifted into a 32-bit mask: no predicates and no
+//      divergent stores in the inner loop.
+//   4. Every lane turns its masks into tile indices (in the shared memory of
+//      the positions, which are done with) and writes its row from them in
+//      16-byte groups of entries.
+// The rows hold the candidates in the order of the cell search, whatever the
+// block shape.
+//
+// Measured on a dam break under way (1.6M particles, 147M entries): 0.764 ms
+// a build, 1.244 ms with a lane per particle walking all 27 cells' candidates
+// and storing single words (32 separate sectors a store); periodic lattice of
+// 1M: 0.625 against 0.942 ms; half2 lists of 0.5M: 0.322 against 0.429 ms.
+// Bound by issue and latency: 54 % of the issue slots with 18 warps an SM, the
+// L1 data pipe (shared memory) at 68 %.
+#pragma once
+#include "sim_tiled.cuh"
+
+namespace wcsph {
+
+constexpr float kFarAway = 1.0e30f;   // position of removed particles in the j-records
+constexpr float kFarTile = -1.0e30f;  // padding of a tile: within no list radius of anything
+constexpr float kFarLane = 3.0e30f;   // idle lanes of a warp
+
+// Bound on r^2 for staging a candidate, relative to R^2: covers the rounding
+// of the box distance.
+constexpr float kCullMargin = 1.00001f;
+
+// Shared memory of one warp (10.9 KB: 20 warps an SM).  The row buffer (16-bit
+// tile indices, one row a lane) takes the place of the positions once they are
+// tested.  Most cells fill one tile and one row buffer (384 candidates and 64
+// indices: 25 warps an SM but 1.27 times the instructions, 0.826 ms; 512 and
+// 128: 16 warps, 0.846 ms).
+constexpr int kScanTile = 448;  // candidates
+struct alignas(16) ScanTile {
+  static constexpr int kBuf = 112;  // indices per row
+  union {
+    float pos[3][kScanTile];
+    uint16_t buf[32][kBuf + 2];  // + 2: the rows start in different banks
+  };
+  uint32_t e[kScanTile];
+  uint32_t mask[kScanTile / 32][32];  // 32 candidates a word
+};
+
+// Minimum / maximum over the warp.
+__device__ __forceinline__ float warp_min_f(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float warp_max_f(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+// Low two bits of a particle's cell coordinates, one nibble per axis, as
+// k_permute leaves them in x0[p].w (half2 entries name the neighbour cell).
+__device__ __forceinline__ uint32_t cell_nibbles(int cx, int cy, int cz) {
+  return (uint32_t)(cx & 3) | ((uint32_t)(cy & 3) << 4) | ((uint32_t)(cz & 3) << 8);
+}
+
+template <bool H16, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_list_scan(const __grid_constant__ StepArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const unsigned full = 0xffffffffu;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  ScanTile& S = reinterpret_cast<ScanTile*>(smem_raw)[warp];
+  float *tx = S.pos[0], *ty = S.pos[1], *tz = S.pos[2];
+  uint32_t* te = S.e;
+  const unsigned lt = lanemask_lt();
+  const int nrun = *a.run_count;
+  const int L = a.list_max;
+  const int ox = lane % 3 - 1, oy = (lane / 3) % 3 - 1, oz = lane / 9 - 1;  // neighbour cell of lane < 27
+  const bool partial = a.inst_keep && a.list_flags[kLfPartial] != 0u;
+  int longest = 0;
+  const int stride = gridDim.x * WARPS;
+  int c = blockIdx.x * WARPS + warp;
+  int lin_next = c < nrun ? a.run_list[c] : 0;
+  for (; c < nrun; c += stride) {
+    const int lin = lin_next;
+    if (c + stride < nrun) lin_next = a.run_list[c + stride];
+    const int s = a.cell_start[lin], e = a.cell_end[lin];
+    const int inst = a.alt.flags[s] & kInstMask;
+    if (partial && a.inst_keep[inst]) continue;  // keeps its lists
+    const InstParams& P = a.params[inst];
+    if (!wants_force(P, a.dyn[inst], a.phase[inst])) {
+      for (int p = s + lane; p < e; p += 32) a.list_cnt[p] = 0;
+      continue;
+    }
+    const int nx = P.ncell[0], ny = P.ncell[1];
+    const int local = lin - P.cell_base;
+    const int cx = local % nx, cy = (local / nx) % ny, cz = local / (nx * ny);
+
+    // the neighbour cells, one per lane, and the runs they form
+    int start = 0, end = 0;
+    float shx = 0.f, shy = 0.f, shz = 0.f;
+    uint32_t image = 13;
+    if (lane < 27) {
+      int x, y, z;
+      if (neighbor_cell(P, 0, cx + ox, x, shx) && neighbor_cell(P, 1, cy + oy, y, shy) &&
+          neighbor_cell(P, 2, cz + oz, z, shz)) {
+        const int l2 = P.cell_base + (z * ny + y) * nx + x;
+        start = a.cell_start[l2];
+        end = a.cell_end[l2];
+        image = (uint32_t)((shx > 0.f) - (shx < 0.f) + 1) + 3u * (uint32_t)((shy > 0.f) - (shy < 0.f) + 1) +
+                9u * (uint32_t)((shz > 0.f) - (shz < 0.f) + 1);
+      }
+    }
+    const unsigned some = __ballot_sync(full, end > start);  // non-empty cells
+    const unsigned before = some & lt;
+    const int prev = before ? 31 - __clz(before) : 0;
+    const int prev_end = __shfl_sync(full, end, prev);
+    const uint32_t prev_image = __shfl_sync(full, image, prev);
+    const bool head = end > start && (!before || prev_end != start || prev_image != image);
+    const unsigned heads = __ballot_sync(full, head);
+    const unsigned later = lane < 31 ? heads >> (lane + 1) : 0u;
+    const int next_head = later ? lane + __ffs(later) : 32;  // first lane of the next run
+    const unsigned upto = next_head < 32 ? some & ((1u << next_head) - 1u) : some;
+    const int run_end = __shfl_sync(full, end, upto ? 31 - __clz(upto) : 0);
+    const uint32_t ci = cell_nibbles(cx, cy, cz);
+    const float R2 = P.HL2, cull = P.HL2 * kCullMargin;
+    const uint32_t hb = __float_as_uint(R2) - 1u;
+    const f2 NR2 = dup(-R2);
+
+    for (int ib = s; ib < e; ib += 32) {
+      const int nbat = min(32, e - ib);
+      const bool mine = lane < nbat;
+      float4 I = make_float4(kFarLane, kFarLane, kFarLane, 0.f);
+      if (mine) I = __ldg(&a.jr[ib + lane].a);
+      // bounding box of the batch's live particles
+      const bool live = mine && I.x < kFarAway;
+      const float big = __int_as_float(0x7f800000);
+      const float bx0 = warp_min_f(live ? I.x : big), bx1 = warp_max_f(live ? I.x : -big);
+      const float by0 = warp_min_f(live ? I.y : big), by1 = warp_max_f(live ? I.y : -big);
+      const float bz0 = warp_min_f(live ? I.z : big), bz1 = warp_max_f(live ? I.z : -big);
+      const f2 IX = dup(I.x), IY = dup(I.y), IZ = dup(I.z);
+      uint32_t* row = a.list + (size_t)(mine ? ib + lane : s) * L;
+      int len = 0;  // entries of this lane's row
+
+      unsigned hm = heads;
+      int qb = 0, q1 = 0;  // the current run's remaining slots
+      float sx = 0.f, sy = 0.f, sz = 0.f;
+      uint32_t im = 0, wrap_mask = 0, wrap_code = 0;
+      do {
+        int tn = 0;                       // staged candidates
+        int own0 = kScanTile, own1 = 0;   // tile indices that hold the cell's own particles
+        while (true) {
+          if (qb >= q1) {  // the next run
+            if (!hm) break;
+            const int h = __ffs(hm) - 1;
+            hm &= hm - 1;
+            qb = __shfl_sync(full, start, h), q1 = __shfl_sync(full, run_end, h);
+            sx = __shfl_sync(full, shx, h), sy = __shfl_sync(full, shy, h), sz = __shfl_sync(full, shz, h);
+            im = __shfl_sync(full, image, h);
+            if (H16) {  // an axis on which the run wraps has one offset; elsewhere the cells' low bits give it
+              wrap_mask = (sx != 0.f ? 0x003u : 0u) | (sy != 0.f ? 0x030u : 0u) | (sz != 0.f ? 0x300u : 0u);
+              wrap_code = (sx > 0.f ? 0x002u : 0u) | (sy > 0.f ? 0x020u : 0u) | (sz > 0.f ? 0x200u : 0u);
+            }
+          }
+          if (tn + 64 > kScanTile) break;
+          float4 J[2];
+          uint32_t cj[2];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const int q = qb + 32 * r + lane;
+            if (q < q1) {
+              J[r] = __ldg(&a.jr[q].a);
+              if (H16) cj[r] = __float_as_uint(__ldg(&a.x0[q].w));
+            }
+          }
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const int q = qb + 32 * r + lane;
+            if (qb + 32 * r < q1) {  // the same for the whole warp
+              const float x = __fadd_rn(J[r].x, sx), y = __fadd_rn(J[r].y, sy), z = __fadd_rn(J[r].z, sz);
+              const float dx = fmaxf(fmaxf(bx0 - x, x - bx1), 0.f), dy = fmaxf(fmaxf(by0 - y, y - by1), 0.f),
+                          dz = fmaxf(fmaxf(bz0 - z, z - bz1), 0.f);
+              const bool in = q < q1 && dx * dx + dy * dy + dz * dz < cull;
+              const unsigned keep = __ballot_sync(full, in);
+              if (in) {
+                uint32_t ent = (uint32_t)q | (im << 27);
+                if (H16) {
+                  uint32_t t = (cj[r] + 0x555u - ci) & 0x333u;  // offset + 1 per axis, no borrow between nibbles
+                  t = (t & ~wrap_mask) | wrap_code;
+                  ent = (uint32_t)q |
+                        (((t & 3u) | ((t >> 2) & 0xcu) | ((t >> 4) & 0x30u)) << kH16SlotBits);
+                }
+                const int u = tn + __popc(keep & lt);
+                tx[u] = x, ty[u] = y, tz[u] = z, te[u] = ent;
+              }
+              if (im == 13u && qb + 32 * r < e && qb + 32 * r + 32 > s) own0 = min(own0, tn), own1 = tn + __popc(keep);
+              tn += __popc(keep);
+            }
+          }
+          qb += 64;
+        }
+        const int tn32 = (tn + 31) & ~31;
+        if (tn + lane < tn32) {
+          tx[tn + lane] = kFarTile, ty[tn + lane] = kFarTile, tz[tn + lane] = kFarTile;
+          te[tn + lane] = 0u;
+        }
+        __syncwarp();
+        for (int u0 = 0; u0 < tn32; u0 += 32) {
+          uint32_t m = 0;
+          if (u0 + 32 <= own0 || u0 >= own1) {
+#pragma unroll
+            for (int u = 0; u < 32; u += 4) {
+              const ulonglong2 X = *reinterpret_cast<const ulonglong2*>(&tx[u0 + u]);
+              const ulonglong2 Y = *reinterpret_cast<const ulonglong2*>(&ty[u0 + u]);
+              const ulonglong2 Z = *reinterpret_cast<const ulonglong2*>(&tz[u0 + u]);
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const f2 DX = sub2(IX, h ? X.y : X.x), DY = sub2(IY, h ? Y.y : Y.x), DZ = sub2(IZ, h ? Z.y : Z.x);
+                // dist2 per half, then r^2 - R^2: negative exactly when r^2 < R^2
+                const f2 T = add2(fma2(DZ, DZ, fma2(DY, DY, mul2(DX, DX))), NR2);
+                m = __funnelshift_l(__float_as_uint(lo(T)), m, 1);
+                m = __funnelshift_l(__float_as_uint(hi(T)), m, 1);
+              }
+            }
+          } else {  // the cell's own particles: 0 < r^2 < R^2 (the particle itself, and any at its very place, out)
+#pragma unroll 4
+            for (int u = 0; u < 32; ++u) {
+              const float r2 = dist2(I.x - tx[u0 + u], I.y - ty[u0 + u], I.z - tz[u0 + u]);
+              m = 2u * m + (__float_as_uint(r2) - 1u < hb ? 1u : 0u);
+            }
+          }
+          S.mask[u0 >> 5][lane] = m;  // bit 31 - u: candidate u0 + u is within the list radius
+        }
+        __syncwarp();
+        const int words = tn32 >> 5;
+        uint16_t* buf = S.buf[lane];
+        for (int w = 0; w < words;) {
+          // as many words as fit every lane's row buffer
+          int n = 0;
+          for (; w < words; ++w) {
+            uint32_t m = S.mask[w][lane];
+            if (__any_sync(full, n + __popc(m) > ScanTile::kBuf)) break;
+            while (m) {
+              const int u = __clz(m);
+              m ^= 0x80000000u >> u;
+              buf[n++] = (uint16_t)(32 * w + u);
+            }
+          }
+          // up to an entry whose place in the row is a multiple of four, then whole groups, then the rest
+          int g = 0;
+          for (; g < n && ((len + g) & 3); ++g)
+            if (len + g < L) row[len + g] = te[buf[g]];
+          for (; g + 4 <= n; g += 4) {
+            const uint4 ent = make_uint4(te[buf[g]], te[buf[g + 1]], te[buf[g + 2]], te[buf[g + 3]]);
+            if (len + g + 4 <= L) *reinterpret_cast<uint4*>(&row[len + g]) = ent;
+          }
+          for (; g < n; ++g)
+            if (len + g < L) row[len + g] = te[buf[g]];
+          len += n;
+        }
+        __syncwarp();
+      } while (hm || qb < q1);
+      if (mine) {
+        a.list_cnt[ib + lane] = len;
+        if (len > L) {
+          a.list_flags[kLfOverflowPending] = 1u;  // the next step rebuilds
+        } else {  // pad the row to a whole group of four (list_max is a multiple of four)
+          for (int k = len; k < ((len + 3) & ~3); ++k) row[k] = a.list_pad;
+        }
+        longest = max(longest, len);
+      }
+    }
+  }
+  longest = __reduce_max_sync(full, longest);
+  if (lane == 0 && longest > 0) atomicMax(&a.list_flags[kLfLongest], (unsigned)longest);
+}
+
+template <bool H16, int WARPS>
+inline int launch_list_scan_v(const StepArgs& a, cudaStream_t s) {
+  static TiledLaunch L[16];
+  int dev = 0;
+  WCSPH_CUDA(cudaGetDevice(&dev));
+  TiledLaunch& T = L[dev & 15];
+  auto kern = k_list_scan<H16, WARPS>;
+  const int bytes = (int)sizeof(ScanTile) * WARPS;
+  if (T.device != dev) {
+    WCSPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    int per_sm = 0, sms = 0;
+    WCSPH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WARPS * 32, bytes));
+    WCSPH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    T.blocks = std::max(1, per_sm) * sms;
+    T.device = dev;
+  }
+  kern<<<T.blocks, WARPS * 32, bytes, s>>>(a);
+  WCSPH_CUDA(cudaGetLastError());
+  return 0;
+}
+
+// Shapes of the list build's scan: warps per block.  3 and 5 repeat shape 0,
+// 4 and 6 shape 2.  All build the same lists.
+constexpr int kBuildShapes = 7;
+constexpr int kBuildShapesTimed = 3;
+
+template <bool H16>
+inline int launch_list_scan(const StepArgs& a, int n, cudaStream_t s, int shape = 0) {
+  if (n > kMaxTiledParticles) {
+    set_error("the tiled path holds at most %d particles per solver (got %d)", kMaxTiledParticles, n);
+    return WCSPH_E_CAPACITY;
+  }
+  switch (shape) {
+    case 1: return launch_list_scan_v<H16, 2>(a, s);
+    case 2: case 4: case 6: return launch_list_scan_v<H16, 8>(a, s);
+    default: return launch_list_scan_v<H16, 4>(a, s);
+  }
+}
+
+}  // namespace wcsph

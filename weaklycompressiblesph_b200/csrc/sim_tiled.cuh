@@ -1,11 +1,10 @@
-// Tiled hydro kernel (WCSPH_PREC_TILED, WCSPH_PREC_HALF2; the two differ only
-// in the entries a list build writes): one warp per non-empty cell.
+// Tiled hydro kernel (WCSPH_PREC_TILED, and WCSPH_PREC_HALF2 without lists):
+// one warp per non-empty cell.
 //
 //   1. The 27 neighbour cells of the warp's cell are flattened into one
 //      candidate list and staged into the warp's shared-memory tile as
 //      structure-of-arrays x[], y[], z[] (pre-shifted by the periodic image)
-//      and e[] (global slot | image code << 27; the half2 list build writes
-//      the neighbour-cell offset code instead), with coalesced loads (a
+//      and e[] (global slot | image code << 27), with coalesced loads (a
 //      cell's particles are contiguous after the sort).
 //   2. The cell's i-particles are taken two at a time.  Each lane tests two
 //      adjacent candidates against both i: one 64-bit shared load yields the
@@ -250,109 +249,7 @@ __device__ __forceinline__ void append2(uint32_t* q, int& n, bool he, bool ho, u
   n += __popc(me) + __popc(mo);
 }
 
-// The 27 neighbour-cell ranges of cell (cx, cy, cz) of instance P, one per
-// lane k < 27 (offset (k%3-1, k/3%3-1, k/9-1)): first slot, count, periodic
-// image shift and entry code (the image code k, or with HL, the half2 list
-// build, the neighbour-cell offset + 1 in two bits per axis: its compact
-// records are relative to the build's cells), the exclusive prefix of the
-// counts over the lanes and, in every lane, their total.
-struct NbRanges {
-  int start, excl, total;
-  float shx, shy, shz;
-  uint32_t code;
-};
-template <bool HL>
-__device__ __forceinline__ NbRanges nb_ranges(const StepArgs& a, const InstParams& P, int cx, int cy, int cz,
-                                              int lane) {
-  const unsigned full = 0xffffffffu;
-  const int nx = P.ncell[0], ny = P.ncell[1];
-  NbRanges R;
-  int cnt = 0;
-  R.start = 0, R.shx = 0.f, R.shy = 0.f, R.shz = 0.f, R.code = 13;
-  if (lane < 27) {
-    int x, y, z;
-    if (neighbor_cell(P, 0, cx + lane % 3 - 1, x, R.shx) && neighbor_cell(P, 1, cy + (lane / 3) % 3 - 1, y, R.shy) &&
-        neighbor_cell(P, 2, cz + lane / 9 - 1, z, R.shz)) {
-      const int l2 = P.cell_base + (z * ny + y) * nx + x;
-      R.start = a.cell_start[l2];
-      cnt = a.cell_end[l2] - R.start;
-      R.code = (uint32_t)((R.shx > 0.f) - (R.shx < 0.f) + 1) + 3u * (uint32_t)((R.shy > 0.f) - (R.shy < 0.f) + 1) +
-               9u * (uint32_t)((R.shz > 0.f) - (R.shz < 0.f) + 1);
-    }
-    if (HL) R.code = (uint32_t)(lane % 3) | ((uint32_t)((lane / 3) % 3) << 2) | ((uint32_t)(lane / 9) << 4);
-  }
-  int incl = cnt;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(full, incl, o);
-    if (lane >= o) incl += t;
-  }
-  R.total = __shfl_sync(full, incl, 31);
-  R.excl = incl - cnt;
-  return R;
-}
-
-// Stage candidates [t0, t0 + tn) of a cell's flattened neighbour ranges into
-// a warp's tile: positions pre-shifted by the periodic image, entries slot |
-// code (at bit 27, or with HL at bit 26), padded to a multiple of 64 with
-// positions that no support test accepts.  Candidate u comes from the last
-// neighbour cell k with excl_k <= u (binary search over lanes 0..26);
-// kStageUnroll independent loads per lane are in flight before any store.
-template <bool HL>
-__device__ __forceinline__ void stage_tile(const StepArgs& a, const NbRanges& R, int t0, int tn, float* tx,
-                                           float* ty, float* tz, uint32_t* te, int lane) {
-  const unsigned full = 0xffffffffu;
-  const int tn64 = (tn + 63) & ~63;
-  for (int ub = t0; ub < t0 + tn; ub += 32 * kStageUnroll) {
-    float4 J[kStageUnroll];
-    int gk[kStageUnroll], kk[kStageUnroll];
-#pragma unroll
-    for (int r = 0; r < kStageUnroll; ++r) {
-      const int u = ub + 32 * r + lane;
-      int k = 0;
-#pragma unroll
-      for (int step = 16; step; step >>= 1) {
-        const int cand = k + step;
-        const int ec = __shfl_sync(full, R.excl, cand < 27 ? cand : 26);
-        if (cand < 27 && ec <= u) k = cand;
-      }
-      const int sk = __shfl_sync(full, R.start, k), ek = __shfl_sync(full, R.excl, k);
-      kk[r] = k;
-      gk[r] = sk + (u - ek);
-      if (u < t0 + tn) J[r] = __ldg(&a.jr[gk[r]].a);
-    }
-#pragma unroll
-    for (int r = 0; r < kStageUnroll; ++r) {
-      const int u = ub + 32 * r + lane;
-      const int k = kk[r];
-      const float sx = __shfl_sync(full, R.shx, k), sy = __shfl_sync(full, R.shy, k), sz = __shfl_sync(full, R.shz, k);
-      const uint32_t ck = __shfl_sync(full, R.code, k) << (HL ? kH16SlotBits : 27);
-      if (u < t0 + tn) {
-        tx[u - t0] = __fadd_rn(J[r].x, sx);
-        ty[u - t0] = __fadd_rn(J[r].y, sy);
-        tz[u - t0] = __fadd_rn(J[r].z, sz);
-        te[u - t0] = (uint32_t)gk[r] | ck;
-      }
-    }
-  }
-  for (int u = tn + lane; u < tn64; u += 32) {  // pad to a multiple of 64: never in support
-    tx[u] = 1.0e30f;
-    ty[u] = 1.0e30f;
-    tz[u] = 1.0e30f;
-    te[u] = 0u;
-  }
-}
-
-// k_hydro_tiled keeps its own copy of the neighbour-range and staging code:
-// written through these helpers it allocated registers differently and
-// spilled in its 4- and 8-warp list-build shapes.
-
-// LB (neighbour-list build): scan only.  The scan keeps the candidates
-// within the list radius 2h + skin and each i's queue is written to its list
-// (list_cnt holds the full count, also past the list's capacity); the pair
-// terms and the epilogue are left to the list pass (k_hydro_list) that
-// follows, as on the steps that reuse the lists.
-template <bool H16, int WARPS, int TILE, bool LB = false>
+template <int WARPS, int TILE>
 __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
   constexpr int kTiledWarps = WARPS;
   constexpr int kTile = TILE;
@@ -381,14 +278,10 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
     const int s = a.cell_start[lin], e = a.cell_end[lin];
     const uint32_t f0 = a.alt.flags[s];
     const int inst = f0 & kInstMask;
-    if (LB && a.inst_keep && a.list_flags[kLfPartial] != 0u && a.inst_keep[inst]) continue;  // keeps its lists
     const InstParams& P = a.params[inst];
     const int ph = a.phase[inst];
     if (!wants_force(P, a.dyn[inst], ph)) {
-      for (int p = s + lane; p < e; p += 32) {
-        if (LB) a.list_cnt[p] = 0;
-        else copy_state(a, p);
-      }
+      for (int p = s + lane; p < e; p += 32) copy_state(a, p);
       continue;
     }
     const int nx = P.ncell[0], ny = P.ncell[1];
@@ -408,9 +301,6 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
         code = (uint32_t)((shx > 0.f) - (shx < 0.f) + 1) + 3u * (uint32_t)((shy > 0.f) - (shy < 0.f) + 1) +
                9u * (uint32_t)((shz > 0.f) - (shz < 0.f) + 1);
       }
-      // the half2 list build writes the neighbour-cell offset instead, two
-      // bits per axis (its compact records are relative to the build's cells)
-      if (H16 && LB) code = (uint32_t)(lane % 3) | ((uint32_t)((lane / 3) % 3) << 2) | ((uint32_t)(lane / 9) << 4);
     }
     int incl = nb_cnt;
 #pragma unroll
@@ -421,12 +311,11 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
     const int T = __shfl_sync(full, incl, 31);
     const int excl = incl - nb_cnt;
     const int own = __shfl_sync(full, excl, 13);  // tile offset of the cell's own particles
-    const float HS = LB ? P.HL2 : P.H2;  // scan bound
+    const float HS = P.H2;  // scan bound
     float dt_cand = 0.f;
     bool dt_valid = false;
     for (int ib = s; ib < e; ib += 32) {
       const int nbat = min(32, e - ib);
-      int lcount = 0;  // LB: list entries written so far for i = ib + lane
 #pragma unroll
       for (int k = 0; k < 6; ++k) res[lane][k] = 0.f;
       for (int t0 = 0; t0 < T; t0 += kTile) {
@@ -459,9 +348,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
             const int u = ub + 32 * r + lane;
             const int k = kk[r];
             const float sx = __shfl_sync(full, shx, k), sy = __shfl_sync(full, shy, k), sz = __shfl_sync(full, shz, k);
-            // entries carry the image code, or for the half2 list pass the
-            // neighbour-cell offset (h16_entry)
-            const uint32_t ck27 = __shfl_sync(full, code, k) << (H16 && LB ? kH16SlotBits : 27);
+            const uint32_t ck27 = __shfl_sync(full, code, k) << 27;
             if (u < t0 + tn) {
               tx[u - t0] = __fadd_rn(J[r].x, sx);
               ty[u - t0] = __fadd_rn(J[r].y, sy);
@@ -504,39 +391,12 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
             append2(qb, nb, has_b && rb0 > 0.0f && rb0 < HS, has_b && rb1 > 0.0f && rb1 < HS, E.x, E.y, lt);
           }
           __syncwarp();
-          if (LB) {  // append this tile pass's queue entries to the lists of ia and ibb
-            const int L = a.list_max;
-            const int oa = __shfl_sync(full, lcount, ii), ob = __shfl_sync(full, lcount, ii + 1);
-            uint32_t* la = a.list + (size_t)ia * L;
-            for (int k = lane; k < na; k += 32)
-              if (oa + k < L) la[oa + k] = qa[k];
-            if (has_b) {
-              uint32_t* lb = a.list + (size_t)ibb * L;
-              for (int k = lane; k < nb; k += 32)
-                if (ob + k < L) lb[ob + k] = qb[k];
-            }
-            if (lane == ii) lcount += na;
-            if (has_b && lane == ii + 1) lcount += nb;
-          }
-          if (!LB) hydro_queues2(a, P, ia, ibb, has_b, IA, IB, qa, na, qb, nb, &res[ii], lane);
+          hydro_queues2(a, P, ia, ibb, has_b, IA, IB, qa, na, qb, nb, &res[ii], lane);
           __syncwarp();
         }
       }
       __syncwarp();
-      if (LB) {
-        if (lane < nbat) {
-          a.list_cnt[ib + lane] = lcount;
-          if (lcount > a.list_max) {
-            a.list_flags[kLfOverflowPending] = 1u;  // the next step rebuilds
-          } else {  // pad the row to a whole group of four (list_max is a multiple of four)
-            uint32_t* row = a.list + (size_t)(ib + lane) * a.list_max;
-            for (int k = lcount; k < ((lcount + 3) & ~3); ++k) row[k] = a.list_pad;
-          }
-        }
-        const int mx = __reduce_max_sync(full, lane < nbat ? lcount : 0);
-        if (lane == 0) atomicMax(&a.list_flags[kLfLongest], (unsigned)mx);
-      }
-      if (!LB && lane < nbat) {
+      if (lane < nbat) {
         const int p = ib + lane;
         const float* r = res[lane];
         const uint32_t fp = a.alt.flags[p];
@@ -551,136 +411,19 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
   if (lane == 0 && pairs) atomicAdd(a.pair_count, pairs);
 }
 
-// List build, lane per particle: a warp per non-empty cell stages the
-// cell's candidates as k_hydro_tiled does (stage_tile); then each lane takes
-// one particle i of the cell and walks the tile eight candidates per step
-// (shared-memory broadcasts, four f32x2 distances), appending each candidate
-// within the list radius (0 < r^2 < (2h + skin)^2) to its own list row.  No
-// ballots and no queues: the entries are those of k_hydro_tiled's scan in the
-// same (candidate) order, so the lists are bit-identical.
-template <int WARPS, int TILE>
-struct ScanSmem {
-  float x[WARPS][TILE], y[WARPS][TILE], z[WARPS][TILE];
-  uint32_t e[WARPS][TILE];
-};
-
-template <bool H16, int WARPS, int TILE>
-__global__ void __launch_bounds__(WARPS * 32) k_list_scan(StepArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  ScanSmem<WARPS, TILE>& S = *reinterpret_cast<ScanSmem<WARPS, TILE>*>(smem_raw);
-  const unsigned full = 0xffffffffu;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* tx = S.x[warp];
-  float* ty = S.y[warp];
-  float* tz = S.z[warp];
-  uint32_t* te = S.e[warp];
-  const int nrun = *a.run_count;
-  const int L = a.list_max;
-  const int stride = gridDim.x * WARPS;
-  int c = blockIdx.x * WARPS + warp;
-  int lin_next = c < nrun ? a.run_list[c] : 0;
-  for (; c < nrun; c += stride) {
-    const int lin = lin_next;
-    if (c + stride < nrun) lin_next = a.run_list[c + stride];
-    const int s = a.cell_start[lin], e = a.cell_end[lin];
-    const int inst = a.alt.flags[s] & kInstMask;
-    if (a.inst_keep && a.list_flags[kLfPartial] != 0u && a.inst_keep[inst]) continue;  // keeps its lists
-    const InstParams& P = a.params[inst];
-    if (!wants_force(P, a.dyn[inst], a.phase[inst])) {
-      for (int p = s + lane; p < e; p += 32) a.list_cnt[p] = 0;
-      continue;
-    }
-    const int nx = P.ncell[0], ny = P.ncell[1];
-    const int local = lin - P.cell_base;
-    const NbRanges R = nb_ranges<H16>(a, P, local % nx, (local / nx) % ny, local / (nx * ny), lane);
-    // 0 < r^2 < (2h + skin)^2 as one unsigned compare of the bit patterns
-    // (r^2 is a sum of squares, never negative or NaN)
-    const uint32_t hb = __float_as_uint(P.HL2) - 1u;
-    for (int ib = s; ib < e; ib += 32) {
-      const int p = ib + lane;
-      const bool mine = p < e;
-      const float4 I = __ldg(&a.jr[mine ? p : s].a);
-      const f2 IX = dup(I.x), IY = dup(I.y), IZ = dup(I.z);
-      uint32_t* row = a.list + (size_t)(mine ? p : s) * L;
-      int cnt = 0;
-      for (int t0 = 0; t0 < R.total; t0 += TILE) {
-        const int tn = min(TILE, R.total - t0);
-        __syncwarp();
-        stage_tile<H16>(a, R, t0, tn, tx, ty, tz, te, lane);
-        __syncwarp();
-        if (mine) {
-          for (int u = 0; u < tn; u += 8) {  // the tile is padded to a multiple of 64
-            const f2* x2 = reinterpret_cast<const f2*>(&tx[u]);
-            const f2* y2 = reinterpret_cast<const f2*>(&ty[u]);
-            const f2* z2 = reinterpret_cast<const f2*>(&tz[u]);
-            const uint4 E0 = *reinterpret_cast<const uint4*>(&te[u]);
-            const uint4 E1 = *reinterpret_cast<const uint4*>(&te[u + 4]);
-            float r2[8];
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-              const f2 DX = sub2(IX, x2[h]), DY = sub2(IY, y2[h]), DZ = sub2(IZ, z2[h]);
-              const f2 R2 = fma2(DZ, DZ, fma2(DY, DY, mul2(DX, DX)));  // == dist2 per half
-              r2[2 * h] = lo(R2), r2[2 * h + 1] = hi(R2);
-            }
-            const uint32_t ev[8] = {E0.x, E0.y, E0.z, E0.w, E1.x, E1.y, E1.z, E1.w};
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              if (__float_as_uint(r2[k]) - 1u < hb) {
-                if (cnt < L) row[cnt] = ev[k];
-                ++cnt;
-              }
-            }
-          }
-        }
-      }
-      if (mine) {
-        a.list_cnt[p] = cnt;
-        if (cnt > L) {
-          a.list_flags[kLfOverflowPending] = 1u;  // the next step rebuilds
-        } else {  // pad the row to a whole group of four (list_max is a multiple of four)
-          for (int k = cnt; k < ((cnt + 3) & ~3); ++k) row[k] = a.list_pad;
-        }
-      }
-      const int mx = __reduce_max_sync(full, mine ? cnt : 0);
-      if (lane == 0) atomicMax(&a.list_flags[kLfLongest], (unsigned)mx);
-    }
-  }
-}
-
 struct TiledLaunch {
   int device = -1;
   int blocks = 0;
 };
 
-template <bool H16, int WARPS, int TILE, bool LB>
+template <int WARPS, int TILE>
 inline int launch_pair_tiled_v(const StepArgs& a, cudaStream_t s) {
   static TiledLaunch L[16];
   int dev = 0;
   WCSPH_CUDA(cudaGetDevice(&dev));
   TiledLaunch& T = L[dev & 15];
-  auto kern = k_hydro_tiled<H16, WARPS, TILE, LB>;
+  auto kern = k_hydro_tiled<WARPS, TILE>;
   const int bytes = (int)sizeof(TiledSmem<WARPS, TILE>);
-  if (T.device != dev) {
-    WCSPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    int per_sm = 0, sms = 0;
-    WCSPH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WARPS * 32, bytes));
-    WCSPH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    T.blocks = std::max(1, per_sm) * sms;
-    T.device = dev;
-  }
-  kern<<<T.blocks, WARPS * 32, bytes, s>>>(a);
-  WCSPH_CUDA(cudaGetLastError());
-  return 0;
-}
-
-template <bool H16, int WARPS, int TILE>
-inline int launch_list_scan_v(const StepArgs& a, cudaStream_t s) {
-  static TiledLaunch L[16];
-  int dev = 0;
-  WCSPH_CUDA(cudaGetDevice(&dev));
-  TiledLaunch& T = L[dev & 15];
-  auto kern = k_list_scan<H16, WARPS, TILE>;
-  const int bytes = (int)sizeof(ScanSmem<WARPS, TILE>);
   if (T.device != dev) {
     WCSPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
     int per_sm = 0, sms = 0;
@@ -699,31 +442,16 @@ inline int launch_list_scan_v(const StepArgs& a, cudaStream_t s) {
 // order of any sum, so results are bit-identical whichever is chosen.
 constexpr int kTileShapes = 3;
 
-template <bool H16, bool LB = false>
 inline int launch_hydro_tiled(const StepArgs& a, int n, cudaStream_t s, int shape = 0) {
   if (n > kMaxTiledParticles) {
     set_error("the tiled path holds at most %d particles per solver (got %d)", kMaxTiledParticles, n);
     return WCSPH_E_CAPACITY;
   }
-  if constexpr (LB) {  // list builds only: smaller tiles, more warps per SM (the scan writes no sums)
-    if (shape == 3) return launch_pair_tiled_v<H16, 4, 256, LB>(a, s);
-    if (shape == 4) return launch_pair_tiled_v<H16, 8, 256, LB>(a, s);
-    if (shape == 5) return launch_list_scan_v<H16, 4, 512>(a, s);
-    if (shape == 6) return launch_list_scan_v<H16, 8, 256>(a, s);
-  }
   switch (shape) {
-    case 1: return launch_pair_tiled_v<H16, 2, 512, LB>(a, s);
-    case 2: return launch_pair_tiled_v<H16, 8, 512, LB>(a, s);
-    default: return launch_pair_tiled_v<H16, 4, 512, LB>(a, s);
+    case 1: return launch_pair_tiled_v<2, 512>(a, s);
+    case 2: return launch_pair_tiled_v<8, 512>(a, s);
+    default: return launch_pair_tiled_v<4, 512>(a, s);
   }
 }
-
-// Shapes of the list build's scan-only pass: the three above and two with
-// 256-candidate tiles (half the shared memory a warp, so up to twice the
-// warps per SM; a cell's candidates then take two tile passes, which changes
-// only the order in which its list entries are found within each pass), and
-// the lane-per-particle scan k_list_scan with 4 warps x 512 or 8 warps x 256
-// candidates (the same entries in the same order).
-constexpr int kBuildShapes = 7;
 
 }  // namespace wcsph
