@@ -24,6 +24,7 @@
 #include "sim_scan.cuh"
 #include "sim_slab.cuh"
 #include "sim_list.cuh"
+#include "sim_read.cuh"
 
 namespace wcsph {
 
@@ -54,7 +55,7 @@ struct SimImpl {
   int* d_phase = nullptr;
   int* d_n_alive = nullptr;
   int* run_list = nullptr;
-  int* d_counters = nullptr;  // [0] run_count, [4] density pass in this launch (slab pack: [0..3] between passes)
+  int* d_counters = nullptr;  // [0] run_count, [4] density pass in this launch (slab pack: [0..3], reads: [1], between passes)
   unsigned long long* d_pairs = nullptr;
   double* d_cons = nullptr;
   float4* diag_acc = nullptr;
@@ -95,6 +96,8 @@ struct SimImpl {
   bool lists_valid = false;           // false: the next step is asked to build (kLfForce)
   int kernels_reuse = 0;
   long long steps_launched = 0;
+  ReadRing ring;
+  std::mutex read_mu;                 // reads of one solver share its scratch and ring
 };
 
 constexpr int kListMax = kListMaxEntries;  // entries per particle list (2h + 0.3 h holds ~100-115 at h = 1.3 dx)
@@ -866,6 +869,7 @@ int wcsph_sim_destroy(wcsph_sim* sim) {
   if (S.gexec) cudaGraphExecDestroy(S.gexec);
   for (void* p : S.allocs) cudaFree(p);
   if (S.h_lflags) cudaFreeHost(S.h_lflags);
+  S.ring.release();
   for (cudaEvent_t e : S.step_ev)
     if (e) cudaEventDestroy(e);
   cudaEventDestroy(S.ev0);
@@ -1358,8 +1362,27 @@ int wcsph_sim_instance_status(wcsph_sim* sim, int32_t slot, double* time, int64_
 }  // extern "C"
 
 namespace wcsph {
-// Copy the instance's slice [range_lo, range_hi) of `src` arrays to host in
-// original order.  Extra tail particles (dead, not yet compacted) are scanned too.
+// An instance whose particle ids all have a place in the per-particle scratch
+// is put in order on the device (sim_read.cuh).  A slab's ids run over the whole
+// decomposed simulation and its own particles are few of them: its slots cross
+// as they lie and the host places them.
+static bool read_on_device(const SimImpl& S, int slot) { return !S.inst[slot].slab && S.inst[slot].n <= S.opt.max_particles; }
+
+// The index of a read in the spare buffer set (free between passes), the count
+// of particles without a slot zeroed.
+static int enqueue_read_index(SimImpl& S, int slot, int tail) {
+  unsigned* idx = reinterpret_cast<unsigned*>(S.buf_alt.pid);
+  WCSPH_CUDA(cudaMemsetAsync(S.d_counters + 1, 0, sizeof(int), S.s));
+  WCSPH_CUDA(cudaMemsetAsync(idx, 0, sizeof(unsigned) * (size_t)S.inst[slot].n, S.s));
+  if (S.n_host > 0)
+    k_read_index<<<nblk(S.n_host), kBlock, 0, S.s>>>(S.buf_main, S.d_dyn, S.d_n_alive, S.n_host, slot, S.inst[slot].n,
+                                                     tail, idx);
+  WCSPH_CUDA(cudaGetLastError());
+  return 0;
+}
+
+// A slab's slice [range_lo, range_hi) of the state in slot order.  Extra tail
+// particles (dead, not yet compacted) are scanned too.
 static int read_slice(SimImpl& S, int slot, const SimArrays& A, InstDyn& d, std::vector<float4>& pos,
                       std::vector<float4>& vel, std::vector<float4>& acc, std::vector<int>& pid,
                       std::vector<uint32_t>& flags) {
@@ -1404,6 +1427,23 @@ int wcsph_sim_read_instance(wcsph_sim* sim, int32_t slot, float* pos3, float* ve
     return WCSPH_E_INVALID;
   }
   WCSPH_CUDA(cudaSetDevice(S.opt.device));
+  if (read_on_device(S, slot)) {
+    const int n = S.inst[slot].n;
+    if (n == 0) {
+      WCSPH_CUDA(cudaStreamSynchronize(S.s));
+      return 0;
+    }
+    std::lock_guard<std::mutex> lk(S.read_mu);
+    if (int rc = enqueue_read_index(S, slot, 1)) return rc;
+    float *p3 = (float*)S.buf_alt.pos, *v3 = (float*)S.buf_alt.vel, *a3 = (float*)S.buf_alt.acc;
+    float *rho = (float*)S.buf_alt.vh, *div = rho + n;
+    uint8_t* cover = (uint8_t*)S.buf_alt.flags;
+    k_read_state<<<nblk(n), kBlock, 0, S.s>>>(S.buf_main, (const unsigned*)S.buf_alt.pid, n, p3, v3, a3, rho, div, cover,
+                                              S.d_counters + 1);
+    WCSPH_CUDA(cudaGetLastError());
+    const ReadField f[] = {{p3, pos3, 3}, {v3, vel3, 3}, {rho, dens, 1}, {a3, acc3, 3}, {div, div_v, 1}, {nullptr, dt_i, 1}};
+    return S.ring.copy_out(S.s, n, S.opt.max_particles, cover, S.d_counters + 1, f, 6, alive);
+  }
   std::vector<float4> pos, vel, acc;
   std::vector<int> pid;
   std::vector<uint32_t> flags;
@@ -1434,6 +1474,24 @@ namespace wcsph {
 // The diagnostic arrays of a probe pass over instance slot, in original order.
 static int read_probe(SimImpl& S, int slot, float* acc3, float* div_v, float* dt_i, float* dens_out,
                       int32_t* n_neighbors) {
+  if (read_on_device(S, slot)) {
+    const int n = S.inst[slot].n;
+    if (n == 0) {
+      WCSPH_CUDA(cudaStreamSynchronize(S.s));
+      return 0;
+    }
+    std::lock_guard<std::mutex> lk(S.read_mu);
+    if (int rc = enqueue_read_index(S, slot, 0)) return rc;
+    float *a3 = (float*)S.buf_alt.acc, *div = (float*)S.buf_alt.vh, *dt = div + n, *rho = dt + n;
+    int* nbr = reinterpret_cast<int*>(rho + n);
+    uint8_t* cover = (uint8_t*)S.buf_alt.flags;
+    k_read_diag<<<nblk(n), kBlock, 0, S.s>>>(S.diag_acc, S.diag_dt, S.diag_rho, S.diag_nbr, S.buf_main.flags,
+                                             (const unsigned*)S.buf_alt.pid, n, a3, div, dt, rho, nbr, cover,
+                                             S.d_counters + 1);
+    WCSPH_CUDA(cudaGetLastError());
+    const ReadField f[] = {{a3, acc3, 3}, {div, div_v, 1}, {dt, dt_i, 1}, {rho, dens_out, 1}, {nbr, n_neighbors, 1}};
+    return S.ring.copy_out(S.s, n, S.opt.max_particles, cover, S.d_counters + 1, f, 5, nullptr);
+  }
   WCSPH_CUDA(cudaStreamSynchronize(S.s));
   InstDyn d;
   WCSPH_CUDA(cudaMemcpy(&d, S.d_dyn + slot, sizeof(InstDyn), cudaMemcpyDeviceToHost));
