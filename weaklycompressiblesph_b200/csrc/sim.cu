@@ -22,6 +22,7 @@
 #include "sim_aux.cuh"
 #include "sim_tiled.cuh"
 #include "sim_scan.cuh"
+#include "sim_plain.cuh"
 #include "sim_slab.cuh"
 #include "sim_list.cuh"
 #include "sim_read.cuh"
@@ -279,13 +280,13 @@ static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, 
     // scan reads positions only, and the EoS records it gathers do not enter
     // the lists.  Other passes search the cells for the density.
     if (density && !build_lists) {
-      k_density_plain<<<nblk(n), kBlock, 0, S.s>>>(a);
+      if (int rc = launch_cell_plain<PLAIN_DENSITY>(a, n, S.s)) return rc;
       k_eos<<<nblk(n), kBlock, 0, S.s>>>(a);
       L += 2;
     }
     if (ev) WCSPH_CUDA(cudaEventRecord(ev[2], S.s));
     if (S.opt.precision == WCSPH_PREC_FP32) {
-      k_hydro_plain<true><<<nblk(n), kBlock, 0, S.s>>>(a);
+      if (int rc = launch_cell_plain<PLAIN_HYDRO>(a, n, S.s)) return rc;
     } else if (build_lists) {  // the scan writes the lists, the list pass sums them
       const bool h16 = S.opt.precision == WCSPH_PREC_HALF2;
       if (int rc = h16 ? launch_list_scan<true>(a, n, S.s, S.build_shape)
@@ -294,9 +295,7 @@ static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, 
       if (ev && S.scan_ev) WCSPH_CUDA(cudaEventRecord(S.scan_ev, S.s));
       if (density) {
         if (int rc = launch_density_list(a, n, S.s, h16)) return rc;
-        StepArgs b = a;  // the particles whose list overflowed: the cell search
-        b.density_overflow_only = 1;
-        k_density_plain<<<nblk(n), kBlock, 0, S.s>>>(b);
+        k_density_overflow<<<nblk(n), kBlock, 0, S.s>>>(a);
         k_eos<<<nblk(n), kBlock, 0, S.s>>>(a);
         L += 3;
       }
@@ -314,7 +313,7 @@ static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, 
     if (init_filter) {
       StepArgs b = a;
       b.init_filter = 1;
-      k_density_plain<<<nblk(n), kBlock, 0, S.s>>>(b);
+      if (int rc = launch_cell_plain<PLAIN_DENSITY>(b, n, S.s)) return rc;
       k_apply_init_filter<<<nblk(n), kBlock, 0, S.s>>>(b);
       L += 2;
     }

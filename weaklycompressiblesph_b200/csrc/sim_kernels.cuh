@@ -145,7 +145,6 @@ struct StepArgs {
   float* jpo;             // P/rho^2 of every slot beside jh (jr[p].a.w, gathered in 4 bytes)
   uint32_t list_pad;      // list entry naming the padding slot (k_list_pad_slot): rows are padded with it
                           // to whole groups of four entries
-  int density_overflow_only;  // k_density_plain of a list build: only the particles whose list overflowed
   int probe_density;      // density pass of a probe launch: 0 none, 1 summation, 2 Shepard
   // diagnostics (probe phase)
   float4* diag_acc;
@@ -371,10 +370,11 @@ __device__ __forceinline__ bool wants_force(const InstParams& P, const InstDyn& 
   return ph == PH_INIT || ph == PH_PROBE || (ph == PH_STEP && d.dt_cur > 0.0f);
 }
 
-// Neighbour-cell iteration shared by the plain kernels.  Calls
-// body(q, J, dx, dy, dz, r2, code) for every in-support j (0 < r2 < (2h)^2,
-// FP32 predicate of the oracle); code is the periodic image code of the tiled
-// kernel's queue entries ((sx+1) + 3 (sy+1) + 9 (sz+1) in units of the box).
+// The cell search of one particle: calls body(q, r2, code) for every in-support
+// j (0 < r2 < (2h)^2, FP32 predicate of the oracle), neighbour cells in the order
+// z, y, x and slots in order within a cell; code is the periodic image code of
+// the tiled kernel's queue entries ((sx+1) + 3 (sy+1) + 9 (sz+1) in units of the
+// box).
 template <typename Body>
 __device__ __forceinline__ void for_each_neighbor(const StepArgs& a, const InstParams& P, float xi, float yi, float zi,
                                                   Body&& body) {
@@ -405,7 +405,7 @@ __device__ __forceinline__ void for_each_neighbor(const StepArgs& a, const InstP
           const float dy = __fsub_rn(yi, __fadd_rn(J.y, sy));
           const float dz = __fsub_rn(zi, __fadd_rn(J.z, sz));
           const float r2 = dist2(dx, dy, dz);
-          if (r2 > 0.0f && r2 < H2) body(q, J, dx, dy, dz, r2, code);
+          if (r2 > 0.0f && r2 < H2) body(q, r2, code);
         }
       }
     }
@@ -413,13 +413,14 @@ __device__ __forceinline__ void for_each_neighbor(const StepArgs& a, const InstP
 }
 
 // ---------------------------------------------------------- density pass
-// Summation rho_i = m sum_j W_ij (self included) or the Shepard filter of
-// force.h:12-29, sum m W / sum (m/rho_j) W, from the pre-filter densities.
-__global__ void k_density_plain(StepArgs a) {
+// Density pass of a list build for the particles whose list overflowed, over
+// the cells (k_density_plain's sums; every other particle reads its list,
+// k_density_list).
+__global__ void k_density_overflow(StepArgs a) {
   if (a.dens_any && !*a.dens_any) return;  // no density pass in this launch
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= *a.n_alive) return;
-  if (a.density_overflow_only && a.list_cnt[p] <= a.list_max) return;  // k_density_list has it
+  if (a.list_cnt[p] <= a.list_max) return;
   const int inst = a.alt.flags[p] & kInstMask;
   const InstParams& P = a.params[inst];
   const int kind = density_kind(a, P, a.dyn[inst], a.phase[inst]);
@@ -432,7 +433,7 @@ __global__ void k_density_plain(StepArgs a) {
   float sum = 0.5f, one = 0.5f / rho_i;  // self term: w(0) = 1/2
   const float iH = P.inv_H;
   const bool shep = kind == 2;
-  for_each_neighbor(a, P, I.x, I.y, I.z, [&](int q, const float4&, float, float, float, float r2, uint32_t) {
+  for_each_neighbor(a, P, I.x, I.y, I.z, [&](int q, float r2, uint32_t) {
     const float w = spline_w(sqrtf(r2) * iH);
     sum += w;
     if (shep) one += w / __ldg(&a.jr[q].b.w);
@@ -547,72 +548,6 @@ __device__ __forceinline__ void copy_state(const StepArgs& a, int p) {
   a.main.acc[p] = a.alt.acc[p];
   a.main.pid[p] = a.alt.pid[p];
   a.main.flags[p] = a.alt.flags[p];
-}
-
-// ------------------------------------------------------------ hydro pass
-// One thread per i-particle (the plain FP32 path).  Restates force.h:38-57
-// for uniform h, m, nu within an instance:
-//   a_i  = m sum_j [ -(P_i/rho_i^2 + P_j/rho_j^2 + Pi_ij) g + 4 nu g r^2 / ((rho_i+rho_j)(r^2+eps h^2)) dv ] ...
-// with gradW = g dr; div v_i = -m/rho_i sum_j g (dr.dv); dt_i = C h / (c_i + v_sig).
-// The epilogue adds gravity (Dam2.h:104-108), does the final kick
-// (class.h:160-163), the density floor (Dam2.h:111), and folds the CFL limits
-// of integral.h:2-12 into the instance's next dt.
-template <bool COUNT>
-__global__ void __launch_bounds__(256) k_hydro_plain(StepArgs a) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = *a.n_alive;
-  const bool in = p < n;
-  int inst = 0;
-  float dt_cand = 0.0f;
-  bool dt_valid = false;
-  unsigned cnt = 0;
-  if (in) {
-    const uint32_t f = a.alt.flags[p];
-    inst = f & kInstMask;
-    const InstParams& P = a.params[inst];
-    const int ph = a.phase[inst];
-    if (wants_force(P, a.dyn[inst], ph)) {
-      const float4 I = a.jr[p].a;
-      const float4 IB = a.jr[p].b;
-      const float ci = a.jC[p];
-      const float rho_i = IB.w, po_i = I.w;
-      float ax = 0.f, ay = 0.f, az = 0.f, dsum = 0.f, vsig = 0.f;
-      const float h = P.h, eh2 = P.eh2, Kg = P.Kg, iH = P.inv_H, alpha = P.alpha, beta = P.beta, nu4 = P.nu4;
-      const int vs = P.vsig_mode;
-      for_each_neighbor(a, P, I.x, I.y, I.z, [&](int q, const float4& J, float dx, float dy, float dz, float r2,
-                                                  uint32_t) {
-        ++cnt;
-        const float4 JB = __ldg(&a.jr[q].b);
-        const float cj = __ldg(&a.jC[q]);
-        const float rinv = rsqrtf(r2);
-        const float g = spline_F(r2 * rinv * iH) * Kg * rinv;
-        const float dvx = IB.x - JB.x, dvy = IB.y - JB.y, dvz = IB.z - JB.z;
-        const float drdv = dx * dvx + dy * dvy + dz * dvz;
-        const float rden = __frcp_rn(r2 + eh2);
-        const float mu = drdv < 0.0f ? h * drdv * rden : 0.0f;
-        const float rs = __frcp_rn(rho_i + JB.w);
-        const float av = (beta * mu - alpha * 0.5f * (ci + cj)) * mu * 2.0f * rs;
-        vsig = vs ? fmaxf(vsig, -mu) : fmaxf(vsig, mu);
-        const float pg = (po_i + J.w + av) * g;
-        const float visc = nu4 * g * r2 * rs * rden;
-        ax += visc * dvx - pg * dx;
-        ay += visc * dvy - pg * dy;
-        az += visc * dvz - pg * dz;
-        dsum += g * drdv;
-      });
-      finish_hydro(a, p, P, inst, ph, f, ax, ay, az, dsum, vsig, cnt, dt_cand, dt_valid);
-      if (f & kGhostBit) cnt = 0;  // pairs are counted for owned particles only
-    } else {
-      copy_state(a, p);
-    }
-  }
-  dt_min(a.dyn, inst, dt_cand, dt_valid);
-  if (COUNT) {
-    unsigned long long c = cnt;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(a.pair_count, c);
-  }
 }
 
 // Dead tail [n_alive, n_host): carry the slots over to main unchanged so that

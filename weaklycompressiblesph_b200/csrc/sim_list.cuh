@@ -250,8 +250,8 @@ __global__ void __launch_bounds__(128) k_density_list(StepArgs a) {
   const float iH = P.inv_H, H2 = P.H2;
   const float4 I = a.jr[p].a;
   const float rho_i = a.jr[p].b.w;
-  // a list that overflowed at this step's build: k_density_plain sums it over
-  // the cell search (density_overflow_only), and the next step builds again
+  // a list that overflowed at this step's build: k_density_overflow sums it over
+  // the cell search (k_density_overflow), and the next step builds again
   if (a.list_cnt[p] > a.list_max) return;
   const int n = min(a.list_cnt[p], a.list_max);
   const uint4* row = reinterpret_cast<const uint4*>(a.list + (size_t)p * a.list_max);
@@ -496,7 +496,7 @@ __device__ __forceinline__ void hydro_list_body(const StepArgs& a) {
         // next step, so no list step ever sees it): sum over the cell search
         // of the build's cell table instead, one j at a time.
         for_each_neighbor(a, P, R.a.x, R.a.y, R.a.z,
-                          [&](int q, const float4&, float, float, float, float, uint32_t code) {
+                          [&](int q, float, uint32_t code) {
                             const JRec Rq = ld_jrec(&a.jr[q]);
                             const float cq = g7 ? lo(snds7_2(dup(Rq.b.w), RHO0, IRHO0, C0)) : __ldg(&a.jC[q]);
                             pair2<false>(P, C, I, Rq, R, code, 13u, dup(cq), true, false, AX, AY, AZ, DS, vsa, vsb,

@@ -1,0 +1,329 @@
+// Density and hydro passes of the plain FP32 path and the density pass of the
+// other searching passes: every particle's neighbours in the order of the cell
+// search (for_each_neighbor), summed one after the other by the particle's lane.
+//
+// One warp per non-empty cell, up to 32 of its particles at a time.  The
+// candidates of the 27 neighbour cells are staged in shared memory with all
+// that a pair needs, runs of slots along x at a time, when they lie within the
+// support radius of the batch's bounding box; every lane tests 32 of them at a
+// time into a bit mask (packed f32x2, the sign of r^2 - H^2), and evaluates the
+// pairs of its masks.  The additions and their order are those of a loop over
+// every candidate, so that the block shape and the staging never change a bit.
+//
+// Against one thread per particle that walked the 27 cells itself, a step's
+// hydro pass: dam break of 12,600 particles 163 -> 41 us, of 54,500 186 -> 80,
+// of 477,000 559 -> 523, of 1.25 M 1395 -> 1356; cells of 83 particles (8,100 in
+// all) 492 -> 370.  Density pass of a lattice of 64,000: 149 -> 81 us.
+// Small solvers are bound by the instructions of one cell's warp (9,000, at six
+// cycles each), large ones by the same stream at 12 warps an SM.  Two candidates'
+// terms are evaluated side by side: one at a time is 570 us at 477,000.  Four
+// warps a batch that rank the candidates and share the terms through shared
+// memory are no faster for small solvers (41 us) and slower for large (943 us).
+#pragma once
+#include "sim_scan.cuh"
+
+namespace wcsph {
+
+enum PlainPass { PLAIN_HYDRO, PLAIN_DENSITY };
+
+constexpr int kBatches = 2;  // blocks that share a cell's batches (hydro pass; most density launches have nothing to do)
+constexpr int kStage = 4;  // groups of 32 candidates whose loads are in flight together
+
+// Shared memory of a warp: 448 candidates (most cells' in one tile).
+template <int PASS>
+struct alignas(16) PlainTile {
+  float pos[3][kScanTile];                                // shifted by the periodic image
+  float4 b[PASS == PLAIN_HYDRO ? kScanTile : 1];          // v, rho
+  float2 pc[PASS == PLAIN_HYDRO ? kScanTile : 1];         // P / rho^2, c
+  float rho[PASS == PLAIN_DENSITY ? kScanTile : 1];
+  uint32_t mask[kScanTile / 32][32];
+};
+
+struct PairConst {
+  float h, eh2, Kg, iH, alpha, beta, nu4;
+};
+struct PairTerm {
+  float x, y, z, g, drdv, mu;
+};
+// Terms of the pair of particle (I, IB, ci) with candidate u; false for the
+// particle itself, and any at its very place.
+__device__ __forceinline__ bool pair_term(const PairConst& C, const float4& I, const float4& IB, float ci, int u,
+                                          const PlainTile<PLAIN_HYDRO>& S, PairTerm& t) {
+  const float dx = __fsub_rn(I.x, S.pos[0][u]), dy = __fsub_rn(I.y, S.pos[1][u]), dz = __fsub_rn(I.z, S.pos[2][u]);
+  const float r2 = dist2(dx, dy, dz);
+  const float4 JB = S.b[u];
+  const float2 pc = S.pc[u];
+  const float rinv = rsqrtf(r2);
+  const float g = spline_F(r2 * rinv * C.iH) * C.Kg * rinv;
+  const float dvx = IB.x - JB.x, dvy = IB.y - JB.y, dvz = IB.z - JB.z;
+  const float drdv = dx * dvx + dy * dvy + dz * dvz;
+  const float rden = __frcp_rn(r2 + C.eh2);
+  const float mu = drdv < 0.0f ? C.h * drdv * rden : 0.0f;
+  const float rs = __frcp_rn(IB.w + JB.w);
+  const float av = (C.beta * mu - C.alpha * 0.5f * (ci + pc.y)) * mu * 2.0f * rs;
+  const float pg = (I.w + pc.x + av) * g;
+  const float visc = C.nu4 * g * r2 * rs * rden;
+  t.x = visc * dvx - pg * dx;
+  t.y = visc * dvy - pg * dy;
+  t.z = visc * dvz - pg * dz;
+  t.g = g;
+  t.drdv = drdv;
+  t.mu = mu;
+  return r2 > 0.0f;
+}
+__device__ __forceinline__ bool density_term(const float4& I, int u, const PlainTile<PLAIN_DENSITY>& S, float iH,
+                                             float& w) {
+  const float r2 = dist2(__fsub_rn(I.x, S.pos[0][u]), __fsub_rn(I.y, S.pos[1][u]), __fsub_rn(I.z, S.pos[2][u]));
+  w = spline_w(sqrtf(r2) * iH);
+  return r2 > 0.0f;
+}
+
+template <int PASS>
+__device__ __forceinline__ void cell_pass(const StepArgs& a, PlainTile<PASS>& S) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x;
+  const unsigned lt = lanemask_lt();
+  float *tx = S.pos[0], *ty = S.pos[1], *tz = S.pos[2];
+  const int nrun = *a.run_count;
+  const int ox = lane % 3 - 1, oy = (lane / 3) % 3 - 1, oz = lane / 9 - 1;  // neighbour cell of lane < 27
+  unsigned long long pairs = 0;
+  for (int k = blockIdx.x; k < nrun; k += gridDim.x) {
+    const int lin = a.run_list[k];
+    const int s = a.cell_start[lin], e = a.cell_end[lin];
+    if (s + 32 * (int)blockIdx.y >= e) continue;  // blockIdx.y: every gridDim.y-th batch of a cell
+    const int inst = a.alt.flags[s] & kInstMask;
+    const InstParams& P = a.params[inst];
+    const int ph = a.phase[inst];
+    const int kind = PASS == PLAIN_DENSITY ? density_kind(a, P, a.dyn[inst], ph) : 0;
+    if (PASS == PLAIN_DENSITY ? !kind : !wants_force(P, a.dyn[inst], ph)) {
+      if (PASS == PLAIN_HYDRO)
+        for (int p = s + 32 * blockIdx.y + lane; p < e; p += 32 * gridDim.y) copy_state(a, p);
+      continue;
+    }
+    const int nx = P.ncell[0], ny = P.ncell[1];
+    const int local = lin - P.cell_base;
+    const int cx = local % nx, cy = (local / nx) % ny, cz = local / (nx * ny);
+
+    // the neighbour cells, one per lane, and the runs they form
+    int start = 0, end = 0;
+    float shx = 0.f, shy = 0.f, shz = 0.f;
+    if (lane < 27) {
+      int x, y, z;
+      if (neighbor_cell(P, 0, cx + ox, x, shx) && neighbor_cell(P, 1, cy + oy, y, shy) &&
+          neighbor_cell(P, 2, cz + oz, z, shz)) {
+        const int l2 = P.cell_base + (z * ny + y) * nx + x;
+        start = a.cell_start[l2];
+        end = a.cell_end[l2];
+      }
+    }
+    const unsigned some = __ballot_sync(full, end > start);  // non-empty cells
+    const unsigned before = some & lt;
+    const int prev = before ? 31 - __clz(before) : 0;
+    const int prev_end = __shfl_sync(full, end, prev);
+    const float px = __shfl_sync(full, shx, prev), py = __shfl_sync(full, shy, prev), pz = __shfl_sync(full, shz, prev);
+    const bool head =
+        end > start && (!before || prev_end != start || px != shx || py != shy || pz != shz);
+    const unsigned heads = __ballot_sync(full, head);
+    const unsigned later = lane < 31 ? heads >> (lane + 1) : 0u;
+    const int next_head = later ? lane + __ffs(later) : 32;  // first lane of the next run
+    const unsigned upto = next_head < 32 ? some & ((1u << next_head) - 1u) : some;
+    const int run_end = __shfl_sync(full, end, upto ? 31 - __clz(upto) : 0);
+    // candidate k of the search lies in the run of the last head whose first <= k, at slot k + its delta
+    int first = head ? run_end - start : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(full, first, o);
+      if (lane >= o) first += t;
+    }
+    const int total = __shfl_sync(full, first, 31);
+    if (head) first -= run_end - start;  // lanes that head no run: first of the run after theirs
+    const int delta = start - first;
+    const float H2 = P.H2, cull = H2 * kCullMargin, iH = P.inv_H;
+    const f2 NH2 = dup(-H2);
+    const PairConst C{P.h, P.eh2, P.Kg, iH, P.alpha, P.beta, P.nu4};
+    const int vs = P.vsig_mode;
+    const bool shep = kind == 2;
+
+    for (int ib = s + 32 * blockIdx.y; ib < e; ib += 32 * gridDim.y) {
+      const int p = ib + lane;
+      const bool mine = p < e;
+      float4 I = make_float4(kFarLane, kFarLane, kFarLane, 0.f), IB = make_float4(0.f, 0.f, 0.f, 1.f);
+      float ci = 0.f;
+      if (mine) {
+        I = a.jr[p].a;
+        IB = a.jr[p].b;
+        if (PASS == PLAIN_HYDRO) ci = a.jC[p];
+      }
+      const float big = __int_as_float(0x7f800000);
+      const float bx0 = warp_min_f(mine ? I.x : big), bx1 = warp_max_f(mine ? I.x : -big);
+      const float by0 = warp_min_f(mine ? I.y : big), by1 = warp_max_f(mine ? I.y : -big);
+      const float bz0 = warp_min_f(mine ? I.z : big), bz1 = warp_max_f(mine ? I.z : -big);
+      const f2 IX = dup(I.x), IY = dup(I.y), IZ = dup(I.z);
+      const float rho_i = IB.w;
+      float ax = 0.f, ay = 0.f, az = 0.f, dsum = 0.f, vsig = 0.f;
+      float sum = 0.5f, one = 0.5f / rho_i;  // self term: w(0) = 1/2
+      unsigned cnt = 0;
+
+      int k0 = 0;  // candidates staged or culled so far
+      do {
+        int tn = 0;  // staged candidates
+        for (; k0 < total && tn + 32 * kStage <= kScanTile; k0 += 32 * kStage) {
+          float4 J[kStage], B[kStage];
+          float c[kStage], sx[kStage], sy[kStage], sz[kStage];
+#pragma unroll
+          for (int r = 0; r < kStage; ++r) {
+            const int k = k0 + 32 * r + lane;
+            int run = 0;  // the last lane with first <= k: the run's head
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+              if (__shfl_sync(full, first, run + o) <= k) run += o;
+            const int q = k + __shfl_sync(full, delta, run);
+            sx[r] = __shfl_sync(full, shx, run), sy[r] = __shfl_sync(full, shy, run), sz[r] = __shfl_sync(full, shz, run);
+            if (k < total) {
+              J[r] = __ldg(&a.jr[q].a);
+              if (PASS == PLAIN_HYDRO || shep) B[r] = __ldg(&a.jr[q].b);
+              if (PASS == PLAIN_HYDRO) c[r] = __ldg(&a.jC[q]);
+            }
+          }
+#pragma unroll
+          for (int r = 0; r < kStage; ++r) {
+            const float x = __fadd_rn(J[r].x, sx[r]), y = __fadd_rn(J[r].y, sy[r]), z = __fadd_rn(J[r].z, sz[r]);
+            const float dx = fmaxf(fmaxf(bx0 - x, x - bx1), 0.f), dy = fmaxf(fmaxf(by0 - y, y - by1), 0.f),
+                        dz = fmaxf(fmaxf(bz0 - z, z - bz1), 0.f);
+            const bool in = k0 + 32 * r + lane < total && dx * dx + dy * dy + dz * dz < cull;
+            const unsigned keep = __ballot_sync(full, in);
+            if (in) {
+              const int u = tn + __popc(keep & lt);
+              tx[u] = x, ty[u] = y, tz[u] = z;
+              if (PASS == PLAIN_HYDRO) S.b[u] = B[r], S.pc[u] = make_float2(J[r].w, c[r]);
+              else if (shep) S.rho[u] = B[r].w;
+            }
+            tn += __popc(keep);
+          }
+        }
+        const int tn32 = (tn + 31) & ~31;
+        if (tn + lane < tn32) tx[tn + lane] = kFarTile, ty[tn + lane] = kFarTile, tz[tn + lane] = kFarTile;
+        __syncwarp();
+        int n = 0;  // this lane's candidates
+        for (int u0 = 0; u0 < tn32; u0 += 32) {
+          uint32_t m = 0;
+#pragma unroll
+          for (int u = 0; u < 32; u += 4) {
+            const ulonglong2 X = *reinterpret_cast<const ulonglong2*>(&tx[u0 + u]);
+            const ulonglong2 Y = *reinterpret_cast<const ulonglong2*>(&ty[u0 + u]);
+            const ulonglong2 Z = *reinterpret_cast<const ulonglong2*>(&tz[u0 + u]);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const f2 DX = sub2(IX, k ? X.y : X.x), DY = sub2(IY, k ? Y.y : Y.x), DZ = sub2(IZ, k ? Z.y : Z.x);
+              const f2 T = add2(fma2(DZ, DZ, fma2(DY, DY, mul2(DX, DX))), NH2);  // negative exactly when r^2 < H^2
+              m = __funnelshift_l(__float_as_uint(lo(T)), m, 1);
+              m = __funnelshift_l(__float_as_uint(hi(T)), m, 1);
+            }
+          }
+          S.mask[u0 >> 5][lane] = m;
+          n += __popc(m);
+        }
+        const int nmax = __reduce_max_sync(full, n);
+        uint32_t m = 0;
+        int w = -1;
+        auto next = [&]() {  // the lane's next candidate
+          while (!m) m = S.mask[++w][lane];
+          const int bit = __clz(m);
+          m ^= 0x80000000u >> bit;
+          return 32 * w + bit;
+        };
+        // two candidates' terms, then their additions in order
+        for (int k = 0; k < nmax; k += 2) {
+          if (k >= n) continue;
+          const int u0 = next(), u1 = k + 1 < n ? next() : -1;
+          if constexpr (PASS == PLAIN_DENSITY) {
+            float w0 = 0.f, w1 = 0.f;
+            const bool b0 = density_term(I, u0, S, iH, w0), b1 = u1 >= 0 && density_term(I, u1, S, iH, w1);
+            if (b0) {
+              sum += w0;
+              if (shep) one += w0 / S.rho[u0];
+            }
+            if (b1) {
+              sum += w1;
+              if (shep) one += w1 / S.rho[u1];
+            }
+          } else {
+            PairTerm t0, t1;
+            const bool b0 = pair_term(C, I, IB, ci, u0, S, t0), b1 = u1 >= 0 && pair_term(C, I, IB, ci, u1, S, t1);
+            if (b0) {
+              ++cnt;
+              ax += t0.x, ay += t0.y, az += t0.z;
+              dsum += t0.g * t0.drdv;
+              vsig = fmaxf(vsig, vs ? -t0.mu : t0.mu);
+            }
+            if (b1) {
+              ++cnt;
+              ax += t1.x, ay += t1.y, az += t1.z;
+              dsum += t1.g * t1.drdv;
+              vsig = fmaxf(vsig, vs ? -t1.mu : t1.mu);
+            }
+          }
+        }
+        __syncwarp();
+      } while (k0 < total);
+      if (PASS == PLAIN_DENSITY) {
+        if (mine) a.rho_new[p] = shep ? sum / one : P.mass * P.Kw * sum;
+      } else {
+        float dt_cand = 0.0f;
+        bool dt_valid = false;
+        if (mine) {
+          const uint32_t f = a.alt.flags[p];
+          finish_hydro(a, p, P, inst, ph, f, ax, ay, az, dsum, vsig, cnt, dt_cand, dt_valid);
+          if (!(f & kGhostBit)) pairs += cnt;  // pairs are counted for owned particles only
+        }
+        dt_min(a.dyn, inst, dt_cand, dt_valid);
+      }
+    }
+  }
+  if (PASS == PLAIN_HYDRO) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(full, pairs, o);
+    if (lane == 0 && pairs) atomicAdd(a.pair_count, pairs);
+  }
+}
+
+// Hydro pass (the plain FP32 path).  Restates force.h:38-57 for uniform h, m,
+// nu within an instance:
+//   a_i  = m sum_j [ -(P_i/rho_i^2 + P_j/rho_j^2 + Pi_ij) g + 4 nu g r^2 / ((rho_i+rho_j)(r^2+eps h^2)) dv ] ...
+// with gradW = g dr; div v_i = -m/rho_i sum_j g (dr.dv); dt_i = C h / (c_i + v_sig).
+// The epilogue adds gravity (Dam2.h:104-108), does the final kick
+// (class.h:160-163), the density floor (Dam2.h:111), and folds the CFL limits
+// of integral.h:2-12 into the instance's next dt.
+__global__ void __launch_bounds__(32, 12) k_hydro_plain(const __grid_constant__ StepArgs a) {
+  __shared__ PlainTile<PLAIN_HYDRO> S;
+  cell_pass<PLAIN_HYDRO>(a, S);
+}
+
+// Summation rho_i = m sum_j W_ij (self included) or the Shepard filter of
+// force.h:12-29, sum m W / sum (m/rho_j) W, from the pre-filter densities.
+__global__ void __launch_bounds__(32, 12) k_density_plain(const __grid_constant__ StepArgs a) {
+  if (a.dens_any && !*a.dens_any) return;  // no density pass in this launch
+  __shared__ PlainTile<PLAIN_DENSITY> S;
+  cell_pass<PLAIN_DENSITY>(a, S);
+}
+
+template <int PASS>
+inline int launch_cell_plain(const StepArgs& a, int n, cudaStream_t s) {
+  static TiledLaunch L[16];
+  int dev = 0;
+  WCSPH_CUDA(cudaGetDevice(&dev));
+  TiledLaunch& T = L[dev & 15];
+  auto kern = PASS == PLAIN_HYDRO ? k_hydro_plain : k_density_plain;
+  if (T.device != dev) {
+    int per_sm = 0, sms = 0;
+    WCSPH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32, 0));
+    WCSPH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    T.blocks = std::max(1, per_sm) * sms;
+    T.device = dev;
+  }
+  kern<<<dim3(std::min(T.blocks, n), PASS == PLAIN_HYDRO ? kBatches : 1), 32, 0, s>>>(a);
+  WCSPH_CUDA(cudaGetLastError());
+  return 0;
+}
+
+}  // namespace wcsph
