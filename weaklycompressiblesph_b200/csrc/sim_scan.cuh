@@ -36,10 +36,6 @@ constexpr float kFarAway = 1.0e30f;   // position of removed particles in the j-
 constexpr float kFarTile = -1.0e30f;  // padding of a tile: within no list radius of anything
 constexpr float kFarLane = 3.0e30f;   // idle lanes of a warp
 
-// Bound on r^2 for staging a candidate, relative to R^2: covers the rounding
-// of the box distance.
-constexpr float kCullMargin = 1.00001f;
-
 // Shared memory of one warp (10.9 KB: 20 warps an SM).  The row buffer (16-bit
 // tile indices, one row a lane) takes the place of the positions once they are
 // tested.  Most cells fill one tile and one row buffer (384 candidates and 64
@@ -55,18 +51,6 @@ struct alignas(16) ScanTile {
   uint32_t e[kScanTile];
   uint32_t mask[kScanTile / 32][32];  // 32 candidates a word
 };
-
-// Minimum / maximum over the warp.
-__device__ __forceinline__ float warp_min_f(float v) {
-  float r;
-  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-  return r;
-}
-__device__ __forceinline__ float warp_max_f(float v) {
-  float r;
-  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-  return r;
-}
 
 // Low two bits of a particle's cell coordinates, one nibble per axis, as
 // k_permute leaves them in x0[p].w (half2 entries name the neighbour cell).

@@ -60,6 +60,22 @@ __device__ __forceinline__ unsigned lanemask_lt() {
   return m;
 }
 
+// Bound on r^2 for staging a candidate, relative to R^2: covers the rounding
+// of the box distance.
+constexpr float kCullMargin = 1.00001f;
+
+// Minimum / maximum over the warp.
+__device__ __forceinline__ float warp_min_f(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float warp_max_f(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
 __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -310,22 +326,25 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
     }
     const int T = __shfl_sync(full, incl, 31);
     const int excl = incl - nb_cnt;
-    const int own = __shfl_sync(full, excl, 13);  // tile offset of the cell's own particles
-    const float HS = P.H2;  // scan bound
+    const float HS = P.H2, cull = HS * kCullMargin;  // scan bound, staging bound
     float dt_cand = 0.f;
     bool dt_valid = false;
     for (int ib = s; ib < e; ib += 32) {
       const int nbat = min(32, e - ib);
 #pragma unroll
       for (int k = 0; k < 6; ++k) res[lane][k] = 0.f;
+      // bounding box of the batch
+      const float4 B = __ldg(&a.jr[ib + min(lane, nbat - 1)].a);
+      const float bx0 = warp_min_f(B.x), bx1 = warp_max_f(B.x), by0 = warp_min_f(B.y), by1 = warp_max_f(B.y),
+                  bz0 = warp_min_f(B.z), bz1 = warp_max_f(B.z);
       for (int t0 = 0; t0 < T; t0 += kTile) {
-        const int tn = min(kTile, T - t0);
-        const int tn64 = (tn + 63) & ~63;
+        const int t1 = min(T, t0 + kTile);
+        int tn = 0;  // staged candidates
         __syncwarp();
         // Flattened staging: candidate u comes from the last neighbour cell k
         // with excl_k <= u (binary search over lanes 0..26); kStageUnroll
         // independent loads per lane are in flight before any store.
-        for (int ub = t0; ub < t0 + tn; ub += 32 * kStageUnroll) {
+        for (int ub = t0; ub < t1; ub += 32 * kStageUnroll) {
           float4 J[kStageUnroll];
           int gk[kStageUnroll], kk[kStageUnroll];
 #pragma unroll
@@ -341,7 +360,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
             const int sk = __shfl_sync(full, nb_start, k), ek = __shfl_sync(full, excl, k);
             kk[r] = k;
             gk[r] = sk + (u - ek);
-            if (u < t0 + tn) J[r] = __ldg(&a.jr[gk[r]].a);
+            if (u < t1) J[r] = __ldg(&a.jr[gk[r]].a);
           }
 #pragma unroll
           for (int r = 0; r < kStageUnroll; ++r) {
@@ -349,14 +368,20 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
             const int k = kk[r];
             const float sx = __shfl_sync(full, shx, k), sy = __shfl_sync(full, shy, k), sz = __shfl_sync(full, shz, k);
             const uint32_t ck27 = __shfl_sync(full, code, k) << 27;
-            if (u < t0 + tn) {
-              tx[u - t0] = __fadd_rn(J[r].x, sx);
-              ty[u - t0] = __fadd_rn(J[r].y, sy);
-              tz[u - t0] = __fadd_rn(J[r].z, sz);
-              te[u - t0] = (uint32_t)gk[r] | ck27;
+            const float x = __fadd_rn(J[r].x, sx), y = __fadd_rn(J[r].y, sy), z = __fadd_rn(J[r].z, sz);
+            const float dx = fmaxf(fmaxf(bx0 - x, x - bx1), 0.f), dy = fmaxf(fmaxf(by0 - y, y - by1), 0.f),
+                        dz = fmaxf(fmaxf(bz0 - z, z - bz1), 0.f);
+            const bool in = u < t1 && dx * dx + dy * dy + dz * dz < cull;
+            const unsigned keep = __ballot_sync(full, in);
+            if (in) {
+              const int v = tn + __popc(keep & lt);
+              tx[v] = x, ty[v] = y, tz[v] = z;
+              te[v] = (uint32_t)gk[r] | ck27;
             }
+            tn += __popc(keep);
           }
         }
+        const int tn64 = (tn + 63) & ~63;
         for (int u = tn + lane; u < tn64; u += 32) {  // pad to a multiple of 64: never in support
           tx[u] = 1.0e30f;
           ty[u] = 1.0e30f;
@@ -368,12 +393,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
           const int ia = ib + ii;
           const bool has_b = ii + 1 < nbat;
           const int ibb = has_b ? ia + 1 : ia;
-          // i positions from the tile when the own cell (lane 13) is staged in this pass
-          const int oa = own + (ia - s) - t0, ob = own + (ibb - s) - t0;
-          const float4 IA = (oa >= 0 && oa < tn) ? make_float4(tx[oa], ty[oa], tz[oa], __ldg(&a.jr[ia].a.w))
-                                                 : __ldg(&a.jr[ia].a);
-          const float4 IB = (ob >= 0 && ob < tn) ? make_float4(tx[ob], ty[ob], tz[ob], __ldg(&a.jr[ibb].a.w))
-                                                 : __ldg(&a.jr[ibb].a);
+          const float4 IA = __ldg(&a.jr[ia].a), IB = __ldg(&a.jr[ibb].a);
           const f2 XA = dup(IA.x), YA = dup(IA.y), ZA = dup(IA.z);
           const f2 XB = dup(IB.x), YB = dup(IB.y), ZB = dup(IB.z);
           int na = 0, nb = 0;
