@@ -50,7 +50,7 @@ template <int WARPS, int TILE>
 struct TiledSmem {
   float x[WARPS][TILE], y[WARPS][TILE], z[WARPS][TILE];  // staged candidates
   uint32_t e[WARPS][TILE];                   // slot | image code << 27
-  uint32_t q[WARPS][2][TILE];                // per-i compacted queues of entries
+  uint16_t q[WARPS][2][TILE];                // per-i compacted queues of tile indices
   float res[WARPS][32][6];                   // per-i accumulators of the current batch
 };
 
@@ -212,16 +212,15 @@ __device__ __forceinline__ void pair2(const InstParams& P, const PairC& C, const
 // Pair terms of i_a (low half) and i_b (high half) over their queues; adds
 // the warp totals into res[0] (i_a) and res[1] (i_b): ax, ay, az, sum g drdv,
 // v_sig, count.  Lanes past a queue's end contribute exactly zero.
-__device__ __forceinline__ void hydro_queues2(const StepArgs& a, const InstParams& P, int ia, int ib, bool has_b,
-                                              const float4& IA, const float4& IBp, const uint32_t* qa, int na,
-                                              const uint32_t* qb, int nb, float (*res)[6], int lane) {
+__device__ __forceinline__ void hydro_queues2(const StepArgs& a, const InstParams& P, const PairC& C, int ia, int ib, bool has_b,
+                                              const float4& IA, const float4& IBp, const uint32_t* te,
+                                              const uint16_t* qa, int na, const uint16_t* qb, int nb, float (*res)[6], int lane) {
   const float4 VA = __ldg(&a.jr[ia].b), VB = __ldg(&a.jr[ib].b);
   PairI I;
   I.X = pk(IA.x, IBp.x), I.Y = pk(IA.y, IBp.y), I.Z = pk(IA.z, IBp.z);
   I.VX = pk(VA.x, VB.x), I.VY = pk(VA.y, VB.y), I.VZ = pk(VA.z, VB.z);
   I.RHO = pk(VA.w, VB.w), I.PO = pk(IA.w, IBp.w);
   I.CI = pk(__ldg(&a.jC[ia]), __ldg(&a.jC[ib]));
-  const PairC C = pair_consts(P);
   const int nbq = has_b ? nb : 0;
   const int n = max(na, nbq);
   f2 AX = 0ull, AY = 0ull, AZ = 0ull, DS = 0ull;
@@ -231,7 +230,7 @@ __device__ __forceinline__ void hydro_queues2(const StepArgs& a, const InstParam
     const bool qva = k < na, qvb = k < nbq;
     // idle halves read i_a's own record (always a valid slot; weight 0 below)
     const uint32_t self = (uint32_t)ia | (13u << 27);
-    const uint32_t ea = qva ? qa[k] : self, eb = qvb ? qb[k] : self;
+    const uint32_t ea = qva ? te[qa[k]] : self, eb = qvb ? te[qb[k]] : self;
     const int ga = ea & kSlotMask, gb = eb & kSlotMask;
     const JRec Ra = ld_jrec(&a.jr[ga]), Rb = ld_jrec(&a.jr[gb]);
     const f2 CJ = pk(__ldg(&a.jC[ga]), __ldg(&a.jC[gb]));
@@ -239,8 +238,8 @@ __device__ __forceinline__ void hydro_queues2(const StepArgs& a, const InstParam
   }
   const float v8[8] = {lo(AX), lo(AY), lo(AZ), -lo(DS), hi(AX), hi(AY), hi(AZ), -hi(DS)};  // DS holds -sum g dr.dv
   const float y = butterfly8(v8, lane);
-  vsa = warp_max(vsa);
-  vsb = warp_max(vsb);
+  vsa = warp_max_f(vsa);
+  vsb = warp_max_f(vsb);
   if ((lane & 3) == 0) {
     const int slot = lane >> 2;
     if (slot < 4) res[0][slot] += y;
@@ -257,11 +256,11 @@ __device__ __forceinline__ void hydro_queues2(const StepArgs& a, const InstParam
 }
 
 // Append the in-support candidates (even/odd halves of the lane's pair) to a queue.
-__device__ __forceinline__ void append2(uint32_t* q, int& n, bool he, bool ho, uint32_t ee, uint32_t eo, unsigned lt) {
+__device__ __forceinline__ void append2(uint16_t* q, int& n, bool he, bool ho, int u, unsigned lt) {
   const unsigned me = __ballot_sync(0xffffffffu, he), mo = __ballot_sync(0xffffffffu, ho);
   const int p = n + __popc(me & lt) + __popc(mo & lt);
-  if (he) q[p] = ee;
-  if (ho) q[p + (he ? 1 : 0)] = eo;
+  if (he) q[p] = (uint16_t)u;
+  if (ho) q[p + (he ? 1 : 0)] = (uint16_t)(u + 1);
   n += __popc(me) + __popc(mo);
 }
 
@@ -277,8 +276,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
   float* ty = S.y[warp];
   float* tz = S.z[warp];
   uint32_t* te = S.e[warp];
-  uint32_t* qa = S.q[warp][0];
-  uint32_t* qb = S.q[warp][1];
+  uint16_t* qa = S.q[warp][0];
+  uint16_t* qb = S.q[warp][1];
   float(*res)[6] = S.res[warp];
   const int nrun = *a.run_count;
   const unsigned lt = lanemask_lt();
@@ -327,6 +326,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
     const int T = __shfl_sync(full, incl, 31);
     const int excl = incl - nb_cnt;
     const float HS = P.H2, cull = HS * kCullMargin;  // scan bound, staging bound
+    const PairC C = pair_consts(P);
     float dt_cand = 0.f;
     bool dt_valid = false;
     for (int ib = s; ib < e; ib += 32) {
@@ -401,17 +401,16 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
             const f2 CX = *reinterpret_cast<const f2*>(&tx[tb]);
             const f2 CY = *reinterpret_cast<const f2*>(&ty[tb]);
             const f2 CZ = *reinterpret_cast<const f2*>(&tz[tb]);
-            const uint2 E = *reinterpret_cast<const uint2*>(&te[tb]);
             f2 DX = sub2(XA, CX), DY = sub2(YA, CY), DZ = sub2(ZA, CZ);
             const f2 RA = fma2(DZ, DZ, fma2(DY, DY, mul2(DX, DX)));  // == dist2 per half
             DX = sub2(XB, CX), DY = sub2(YB, CY), DZ = sub2(ZB, CZ);
             const f2 RB = fma2(DZ, DZ, fma2(DY, DY, mul2(DX, DX)));
             const float ra0 = lo(RA), ra1 = hi(RA), rb0 = lo(RB), rb1 = hi(RB);
-            append2(qa, na, ra0 > 0.0f && ra0 < HS, ra1 > 0.0f && ra1 < HS, E.x, E.y, lt);
-            append2(qb, nb, has_b && rb0 > 0.0f && rb0 < HS, has_b && rb1 > 0.0f && rb1 < HS, E.x, E.y, lt);
+            append2(qa, na, ra0 > 0.0f && ra0 < HS, ra1 > 0.0f && ra1 < HS, tb, lt);
+            append2(qb, nb, has_b && rb0 > 0.0f && rb0 < HS, has_b && rb1 > 0.0f && rb1 < HS, tb, lt);
           }
           __syncwarp();
-          hydro_queues2(a, P, ia, ibb, has_b, IA, IB, qa, na, qb, nb, &res[ii], lane);
+          hydro_queues2(a, P, C, ia, ibb, has_b, IA, IB, te, qa, na, qb, nb, &res[ii], lane);
           __syncwarp();
         }
       }
