@@ -823,7 +823,7 @@ int wcsph_sim_create(const wcsph_sim_options* opt, wcsph_sim** out) {
   S.cub_bytes = cub_sort_bytes((long long)N);
   rc |= alloc(S, &S.cub_tmp, S.cub_bytes);
   if (opt->list_interval > 0) {
-    rc |= alloc(S, (void**)&S.list, N * kListMax * sizeof(uint32_t));
+    rc |= alloc(S, (void**)&S.list, (N + 31) / 32 * 32 * kListMax * sizeof(uint32_t));  // whole groups of 32 rows
     rc |= alloc(S, (void**)&S.list_cnt, N * sizeof(int));
     rc |= alloc(S, (void**)&S.x0, N * sizeof(float4));
     rc |= alloc(S, (void**)&S.d_lflags, kLfWords * sizeof(unsigned));

@@ -153,6 +153,14 @@ struct StepArgs {
   float* diag_rho;
 };
 
+// The neighbour-list row of particle p: group g (entries 4 g to 4 g + 3) at
+// row[32 g].  The rows of 32 consecutive particles are interleaved group by
+// group, so that a warp that walks its particles' rows reads 512 contiguous
+// bytes a group instead of 32 lines.
+__device__ __forceinline__ uint4* list_row(const StepArgs& a, int p) {
+  return reinterpret_cast<uint4*>(a.list) + (size_t)(p >> 5) * (a.list_max * 8) + (p & 31);
+}
+
 __device__ __forceinline__ float bits_f(unsigned b) { return __uint_as_float(b); }
 
 // Density pass of an instance in the current launch: 0 none, 1 summation, 2 Shepard.

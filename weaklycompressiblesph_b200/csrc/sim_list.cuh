@@ -24,6 +24,8 @@
 // without a graph the host reads it.  A displacement beyond skin / 2 at a list
 // step would still set a sticky error that the next wcsph_sim_step reports.
 #pragma once
+#include <type_traits>
+
 #include "sim_tiled.cuh"
 
 namespace wcsph {
@@ -227,6 +229,53 @@ __device__ __forceinline__ void offset_shift(const InstParams& P, const int c[3]
   sx = sh[0], sy = sh[1], sz = sh[2];
 }
 
+// A group of a list row: read once, so past the L1.
+__device__ __forceinline__ uint4 ld_row(const uint4* p) {
+  uint4 e;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(e.x), "=r"(e.y), "=r"(e.z), "=r"(e.w)
+               : "l"(p));
+  return e;
+}
+
+// A thread's way through its list row: every TPI-th group of four entries, in
+// flight kRowStages - 1 groups ahead.  A group's row segment is read once and
+// comes from DRAM, while the loop has few registers to spare, so the groups
+// wait in shared memory (cp.async past the L1, each thread its own 16 bytes: no
+// barrier).  Block of 128 threads.
+constexpr int kRowStages = 4;
+template <int TPI>
+struct RowStream {
+  const uint4* ahead;  // the next group to fetch
+  uint32_t slot;       // shared address of this thread's 16 bytes of stage 0
+  int n;               // entries of the row
+
+  __device__ __forceinline__ void fetch(int k, uint32_t stage) {  // the group at entry k
+    if (k < n)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot + stage), "l"(ahead) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    ahead += 32 * TPI;
+  }
+  __device__ __forceinline__ RowStream(const uint4* row, uint4 (*buf)[128], int n_, int sub)
+      : ahead(row + 32 * sub), n(n_) {
+    slot = (uint32_t)__cvta_generic_to_shared(&buf[0][threadIdx.x]);
+#pragma unroll
+    for (int j = 0; j < kRowStages - 1; ++j) fetch(4 * (sub + TPI * j), j * 2048u);
+  }
+  // The group at entry k = 4 sub, 4 (sub + TPI), ... in turn.
+  __device__ __forceinline__ uint4 get(int k) {
+    const uint32_t stage = (uint32_t)(k / (4 * TPI)) % kRowStages;
+    fetch(k + 4 * TPI * (kRowStages - 1), ((stage + kRowStages - 1) % kRowStages) * 2048u);
+    asm volatile("cp.async.wait_group %0;" ::"n"(kRowStages - 1) : "memory");
+    uint4 e;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(e.x), "=r"(e.y), "=r"(e.z), "=r"(e.w)
+                 : "r"(slot + stage * 2048u)
+                 : "memory");
+    return e;
+  }
+};
+
 // Density pass over the lists: k_density_plain's sums (summation, or the
 // Shepard filter of force.h:12-29) over each particle's list entries that are
 // within the support now, one thread per particle walking its own list row
@@ -254,12 +303,20 @@ __global__ void __launch_bounds__(128) k_density_list(StepArgs a) {
   // the cell search (k_density_overflow), and the next step builds again
   if (a.list_cnt[p] > a.list_max) return;
   const int n = min(a.list_cnt[p], a.list_max);
-  const uint4* row = reinterpret_cast<const uint4*>(a.list + (size_t)p * a.list_max);
+  const uint4* row = list_row(a, p);
+  uint4 next = ld_row(row);  // a group ahead: it comes from DRAM, and the gathers wait for it
   int ci[3] = {0, 0, 0};
-  if (H16 && P.periodic) build_cell(a, P, p, ci);
+  bool wraps = P.periodic;
+  if (H16 && wraps) {  // only particles of the outermost cells have neighbours across a face
+    build_cell(a, P, p, ci);
+    wraps = false;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) wraps |= ci[d] == 0 || ci[d] == P.ncell[d] - 1;
+  }
   float sum = 0.f, one = 0.f;
   for (int k = 0; k < n; k += 4) {
-    const uint4 e4 = __ldg(&row[k >> 2]);
+    const uint4 e4 = next;
+    if (k + 4 < n) next = ld_row(row + 8 * k + 32);
     const uint32_t ent[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -267,9 +324,9 @@ __global__ void __launch_bounds__(128) k_density_list(StepArgs a) {
         const int q = ent[u] & (H16 ? kH16SlotMask : kSlotMask);
         const float4 J = __ldg(&a.jr[q].a);
         float sx = 0.f, sy = 0.f, sz = 0.f;
-        if (P.periodic) {
+        if (wraps) {
           if (H16) offset_shift(P, ci, ent[u], sx, sy, sz);
-          else entry_shift(P, ent[u] >> 27, sx, sy, sz);
+          else if (ent[u] >> 27 != 13u) entry_shift(P, ent[u] >> 27, sx, sy, sz);
         }
         const float dx = __fsub_rn(I.x, __fadd_rn(J.x, sx));
         const float dy = __fsub_rn(I.y, __fadd_rn(J.y, sy));
@@ -487,7 +544,6 @@ __device__ __forceinline__ void hydro_list_body(const StepArgs& a) {
       const f2 RHO0 = dup(P.rho0), IRHO0 = dup(P.inv_rho0), C0 = dup(P.c0);
       const int cnt_build = a.list_cnt[p];
       const int n = cnt_build <= a.list_max ? cnt_build : 0;
-      const uint4* row = reinterpret_cast<const uint4*>(a.list + (size_t)p * a.list_max);
       f2 AX = 0ull, AY = 0ull, AZ = 0ull, DS = 0ull;
       float vsa = 0.f, vsb = 0.f;
       unsigned ca = 0, cb = 0;
@@ -519,8 +575,11 @@ __device__ __forceinline__ void hydro_list_body(const StepArgs& a) {
         H.B = dup(P.B);
         // entries past n up to the end of the group of four name the padding
         // slot, which no support, band or far test accepts
+        const uint4* row = list_row(a, p);
+        uint4 next = ld_row(row + 32 * sub);  // a group ahead: it comes from DRAM, and the gathers wait for it
         for (int k = 4 * sub; k < n; k += 4 * TPI) {
-          const uint4 e = __ldg(&row[k >> 2]);
+          const uint4 e = next;
+          if (k + 4 * TPI < n) next = ld_row(row + 8 * k + 32 * TPI);
           const uint4 Q0 = __ldg(&a.jh[e.x & kH16SlotMask]), Q1 = __ldg(&a.jh[e.y & kH16SlotMask]);
           const uint4 Q2 = __ldg(&a.jh[e.z & kH16SlotMask]), Q3 = __ldg(&a.jh[e.w & kH16SlotMask]);
           h16_pair2<OFT, POR>(a, P, C, I, H, Q0, Q1, e.x, e.y, true, true, g7, RHO0, IRHO0, C0, AX, AY, AZ, DS, vsa,
@@ -532,24 +591,31 @@ __device__ __forceinline__ void hydro_list_body(const StepArgs& a) {
         // idle halves past n read i's own record (weight 0): this loop keeps
         // its selects, which leave the FP32 pass within 96 registers
         const uint32_t self = (uint32_t)p | (13u << 27);
-        for (int k = 4 * sub; k < n; k += 4 * TPI) {
-          const uint4 e = __ldg(&row[k >> 2]);
-          const uint32_t e0 = e.x, e1 = k + 1 < n ? e.y : self, e2 = k + 2 < n ? e.z : self,
-                         e3 = k + 3 < n ? e.w : self;
-          const int g0 = e0 & kSlotMask, g1 = e1 & kSlotMask, g2 = e2 & kSlotMask, g3 = e3 & kSlotMask;
-          const JRec R0 = ld_jrec(&a.jr[g0]), R1 = ld_jrec(&a.jr[g1]);
-          const JRec R2 = ld_jrec(&a.jr[g2]), R3 = ld_jrec(&a.jr[g3]);
-          f2 C01, C23;
-          if (g7) {  // c_j from rho_j: no gather of c
-            C01 = snds7_2(pk(R0.b.w, R1.b.w), RHO0, IRHO0, C0);
-            C23 = snds7_2(pk(R2.b.w, R3.b.w), RHO0, IRHO0, C0);
-          } else {
-            C01 = pk(__ldg(&a.jC[g0]), __ldg(&a.jC[g1])), C23 = pk(__ldg(&a.jC[g2]), __ldg(&a.jC[g3]));
+        __shared__ uint4 s_rows[kRowStages][128];
+        RowStream<TPI> row(list_row(a, p), s_rows, n, sub);
+        auto sum = [&](auto per) {
+          constexpr bool PER = decltype(per)::value;
+          for (int k = 4 * sub; k < n; k += 4 * TPI) {
+            const uint4 e = row.get(k);
+            const uint32_t e0 = e.x, e1 = k + 1 < n ? e.y : self, e2 = k + 2 < n ? e.z : self,
+                           e3 = k + 3 < n ? e.w : self;
+            const int g0 = e0 & kSlotMask, g1 = e1 & kSlotMask, g2 = e2 & kSlotMask, g3 = e3 & kSlotMask;
+            const JRec R0 = ld_jrec(&a.jr[g0]), R1 = ld_jrec(&a.jr[g1]);
+            const JRec R2 = ld_jrec(&a.jr[g2]), R3 = ld_jrec(&a.jr[g3]);
+            f2 C01, C23;
+            if (g7) {  // c_j from rho_j: no gather of c
+              C01 = snds7_2(pk(R0.b.w, R1.b.w), RHO0, IRHO0, C0);
+              C23 = snds7_2(pk(R2.b.w, R3.b.w), RHO0, IRHO0, C0);
+            } else {
+              C01 = pk(__ldg(&a.jC[g0]), __ldg(&a.jC[g1])), C23 = pk(__ldg(&a.jC[g2]), __ldg(&a.jC[g3]));
+            }
+            pair2<true, PER>(P, C, I, R0, R1, e0 >> 27, e1 >> 27, C01, true, k + 1 < n, AX, AY, AZ, DS, vsa, vsb, ca, cb);
+            pair2<true, PER>(P, C, I, R2, R3, e2 >> 27, e3 >> 27, C23, k + 2 < n, k + 3 < n, AX, AY, AZ, DS, vsa, vsb, ca,
+                        cb);
           }
-          pair2<true>(P, C, I, R0, R1, e0 >> 27, e1 >> 27, C01, true, k + 1 < n, AX, AY, AZ, DS, vsa, vsb, ca, cb);
-          pair2<true>(P, C, I, R2, R3, e2 >> 27, e3 >> 27, C23, k + 2 < n, k + 3 < n, AX, AY, AZ, DS, vsa, vsb, ca,
-                      cb);
-        }
+        };
+        if (P.periodic) sum(std::true_type());
+        else sum(std::false_type());
       }
       sx = lo(AX) + hi(AX), sy = lo(AY) + hi(AY), sz = lo(AZ) + hi(AZ), sd = -(lo(DS) + hi(DS));  // DS: -sum g dr.dv
       sv = fmaxf(vsa, vsb);

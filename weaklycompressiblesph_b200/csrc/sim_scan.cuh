@@ -133,7 +133,8 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_list_scan(const __gr
       const float by0 = warp_min_f(live ? I.y : big), by1 = warp_max_f(live ? I.y : -big);
       const float bz0 = warp_min_f(live ? I.z : big), bz1 = warp_max_f(live ? I.z : -big);
       const f2 IX = dup(I.x), IY = dup(I.y), IZ = dup(I.z);
-      uint32_t* row = a.list + (size_t)(mine ? ib + lane : s) * L;
+      uint4* row = list_row(a, mine ? ib + lane : s);
+      auto put = [&](int k, uint32_t ent) { reinterpret_cast<uint32_t*>(row + 32 * (k >> 2))[k & 3] = ent; };
       int len = 0;  // entries of this lane's row
 
       unsigned hm = heads;
@@ -243,13 +244,13 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_list_scan(const __gr
           // up to an entry whose place in the row is a multiple of four, then whole groups, then the rest
           int g = 0;
           for (; g < n && ((len + g) & 3); ++g)
-            if (len + g < L) row[len + g] = te[buf[g]];
+            if (len + g < L) put(len + g, te[buf[g]]);
           for (; g + 4 <= n; g += 4) {
             const uint4 ent = make_uint4(te[buf[g]], te[buf[g + 1]], te[buf[g + 2]], te[buf[g + 3]]);
-            if (len + g + 4 <= L) *reinterpret_cast<uint4*>(&row[len + g]) = ent;
+            if (len + g + 4 <= L) row[8 * (len + g)] = ent;
           }
           for (; g < n; ++g)
-            if (len + g < L) row[len + g] = te[buf[g]];
+            if (len + g < L) put(len + g, te[buf[g]]);
           len += n;
         }
         __syncwarp();
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_list_scan(const __gr
         if (len > L) {
           a.list_flags[kLfOverflowPending] = 1u;  // the next step rebuilds
         } else {  // pad the row to a whole group of four (list_max is a multiple of four)
-          for (int k = len; k < ((len + 3) & ~3); ++k) row[k] = a.list_pad;
+          for (int k = len; k < ((len + 3) & ~3); ++k) put(k, a.list_pad);
         }
         longest = max(longest, len);
       }

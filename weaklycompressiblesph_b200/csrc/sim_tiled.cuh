@@ -126,14 +126,13 @@ struct PairC {
   float H2, iH, KgiH;
   f2 IH, KG3, EH2, HH, NNU4, BETA2, MALPHA;
   int vs;
-  bool per;
 };
 __device__ __forceinline__ PairC pair_consts(const InstParams& P) {
   PairC c;
   c.H2 = P.H2, c.iH = P.inv_H, c.KgiH = P.Kg * P.inv_H;
   c.IH = dup(P.inv_H), c.KG3 = dup(3.0f * P.Kg), c.EH2 = dup(P.eh2), c.HH = dup(P.h);
   c.NNU4 = dup(-P.nu4), c.BETA2 = dup(2.0f * P.beta), c.MALPHA = dup(-P.alpha);
-  c.vs = P.vsig_mode, c.per = P.periodic;
+  c.vs = P.vsig_mode;
   return c;
 }
 
@@ -185,15 +184,16 @@ __device__ __forceinline__ void pair_terms2(const PairC& C, const PairI& I, f2 D
 // Pair terms of two (i, j) pairs at once from FP32 j-records Ra, Rb with
 // image codes ea, eb (entry >> 27) and sound speeds CJ; qva, qvb say whether a
 // half holds a pair (idle halves must still name a valid record; they add
-// exactly zero).  CHECK: halves outside 0 < r^2 < (2h)^2 add exactly zero,
+// exactly zero).  PER: pairs may cross a face of a periodic box (codes other
+// than 13); few do, and their images cost as much as a third of the pair.  CHECK: halves outside 0 < r^2 < (2h)^2 add exactly zero,
 // and na, nb count the halves summed.
-template <bool CHECK>
+template <bool CHECK, bool PER = true>
 __device__ __forceinline__ void pair2(const InstParams& P, const PairC& C, const PairI& I, const JRec& Ra,
                                       const JRec& Rb, uint32_t ea, uint32_t eb, f2 CJ, bool qva, bool qvb, f2& AX,
                                       f2& AY, f2& AZ, f2& DS, float& vsa, float& vsb, unsigned& na, unsigned& nb) {
   const float4 &Ja = Ra.a, &Jb = Rb.a, &JBa = Ra.b, &JBb = Rb.b;
   float jxa = Ja.x, jya = Ja.y, jza = Ja.z, jxb = Jb.x, jyb = Jb.y, jzb = Jb.z;
-  if (C.per) {  // the same rounded image position the scan tested
+  if (PER && (ea != 13u || eb != 13u)) {  // the same rounded image position the scan tested
     float sx, sy, sz;
     entry_shift(P, ea, sx, sy, sz);
     jxa = __fadd_rn(jxa, sx), jya = __fadd_rn(jya, sy), jza = __fadd_rn(jza, sz);
