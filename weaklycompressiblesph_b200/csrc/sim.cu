@@ -465,7 +465,10 @@ static int autotune(SimImpl& S) {
     float best_list = 1e30f;
     const int fixed_list = S.opt.list_shape & 0xff, fixed_build = (S.opt.list_shape >> 8) & 0xff;
     int best_list_shape = fixed_list > 0 ? fixed_list - 1 : 0;
-    for (int v = 0; v < kListShapes && fixed_list == 0; ++v) {
+    int sms = 0;
+    WCSPH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S.opt.device));
+    for (int v : list_shape_candidates(n, h16, sms)) {
+      if (fixed_list > 0) break;
       int rc = time_launches(S, 3, [&]() {
         return h16 ? launch_hydro_list<true>(b, n, S.s, v) : launch_hydro_list<false>(b, n, S.s, v);
       }, &ms);
