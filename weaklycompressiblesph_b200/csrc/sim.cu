@@ -204,6 +204,7 @@ static StepArgs make_args(SimImpl& S) {
   a.pair_count = S.d_pairs;
   a.run_list = S.run_list;
   a.run_count = S.d_counters;
+  a.cells = S.total_cells;
   a.dens_any = S.d_counters + 4;
   a.diag_acc = S.diag_acc;
   a.diag_dt = S.diag_dt;
@@ -242,7 +243,10 @@ __global__ void k_begin_build(StepArgs a) {
     a.dyn[k].range_lo = 0x7fffffff;
     a.dyn[k].range_hi = 0;
   }
-  if (k == 0) *a.n_alive = a.n_host;
+  if (k == 0) {
+    *a.n_alive = a.n_host;
+    *a.run_count = 0;
+  }
 }
 
 static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, int* launches,
@@ -256,8 +260,7 @@ static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, 
     k_begin_build<<<nblk(std::max<int>(1, (int)S.inst.size())), kBlock, 0, S.s>>>(a);
   } else {
     if (ev) WCSPH_CUDA(cudaEventRecord(ev[0], S.s));
-    WCSPH_CUDA(cudaMemsetAsync(S.d_counters + 4, 0, sizeof(int), S.s));
-    k_step_begin<<<nblk(std::max<int>(1, (int)S.inst.size())), kBlock, 0, S.s>>>(a);
+    k_step_begin<<<1, kBlock, 0, S.s>>>(a);
   }
   ++L;
   if (n > 0) {
@@ -267,11 +270,6 @@ static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, 
     WCSPH_CUDA(cub::DeviceRadixSort::SortPairs(S.cub_tmp, bytes, S.keys_in, S.keys_out, S.vals_in, S.vals_out, n, 0,
                                                S.key_bits, S.s));
     L += 2 * ((S.key_bits + 7) / 8) + 1;  // onesweep: histogram + one pass per digit (approximate)
-    if (S.total_cells > 0) {
-      WCSPH_CUDA(cudaMemsetAsync(S.cell_start, 0, sizeof(int) * S.total_cells, S.s));
-      WCSPH_CUDA(cudaMemsetAsync(S.cell_end, 0, sizeof(int) * S.total_cells, S.s));
-    }
-    WCSPH_CUDA(cudaMemsetAsync(S.d_counters, 0, sizeof(int), S.s));
     k_permute<<<nblk(n), kBlock, 0, S.s>>>(a);
     ++L;
     if (ev) WCSPH_CUDA(cudaEventRecord(ev[1], S.s));
@@ -308,8 +306,6 @@ static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, 
     }
     ++L;
     if (ev) WCSPH_CUDA(cudaEventRecord(ev[3], S.s));
-    k_copy_dead<<<nblk(n), kBlock, 0, S.s>>>(a);
-    ++L;
     if (init_filter) {
       StepArgs b = a;
       b.init_filter = 1;
@@ -608,19 +604,16 @@ static int read_list_flags(SimImpl& S) {
   return 0;
 }
 
-// The prologue of a list-mode step: dt rotation (k_step_begin, keeping the
-// build's order), then the device's build decision (k_list_set), which sets
-// the condition `cond` when use_cond.
+// The prologue of a list-mode step: dt rotation and the device's build decision
+// (k_list_set), which sets the condition `cond` when use_cond.
 static int enqueue_list_prologue(SimImpl& S, const StepArgs& a0, cudaGraphConditionalHandle cond, bool use_cond,
                                  cudaEvent_t* ev) {
   StepArgs a = a0;
   a.list_reuse = 1;
   a.x0 = S.x0;
   if (ev) WCSPH_CUDA(cudaEventRecord(ev[0], S.s));
-  WCSPH_CUDA(cudaMemsetAsync(S.d_pairs, 0, sizeof(unsigned long long), S.s));
-  WCSPH_CUDA(cudaMemsetAsync(S.d_counters + 4, 0, sizeof(int), S.s));
-  k_step_begin<<<nblk(std::max<int>(1, (int)S.inst.size())), kBlock, 0, S.s>>>(a);
-  k_list_set<<<1, 1, 0, S.s>>>(a, S.opt.list_interval, cond, use_cond ? 1 : 0);
+  a.zero_pairs = 1;
+  k_list_set<<<1, kBlock, 0, S.s>>>(a, S.opt.list_interval, cond, use_cond ? 1 : 0);
   WCSPH_CUDA(cudaGetLastError());
   return 0;
 }
@@ -732,8 +725,8 @@ static int capture_list_graph(SimImpl& S) {
   const cudaError_t ei = cudaGraphInstantiate(&S.gexec, g, 0);
   cudaGraphDestroy(g);
   if (ei != cudaSuccess) return cuda_fail(ei, "cudaGraphInstantiate (list step)", __FILE__, __LINE__);
-  S.kernels_per_step += 2;  // the prologue's kernels
-  S.kernels_reuse += 2;
+  S.kernels_per_step += 1;  // the prologue's kernel
+  S.kernels_reuse += 1;
   S.graph_dirty = false;
   return 0;
 }
@@ -1320,7 +1313,7 @@ int wcsph_sim_step(wcsph_sim* sim, int32_t nsteps) {
     }
     cudaGraph_t g;
     WCSPH_CUDA(cudaStreamBeginCapture(S.s, cudaStreamCaptureModeThreadLocal));
-    WCSPH_CUDA(cudaMemsetAsync(S.d_pairs, 0, sizeof(unsigned long long), S.s));
+    a.zero_pairs = 1;
     int rc = enqueue_pass(S, a, S.any_density, false, &S.kernels_per_step);
     cudaError_t e = cudaStreamEndCapture(S.s, &g);
     if (rc) return rc;
@@ -1533,9 +1526,8 @@ static int enqueue_probe_lists(SimImpl& S, int density_pass) {
   a.x0 = S.x0;
   a.alt = a.main;
   const int n = S.n_host;
-  WCSPH_CUDA(cudaMemsetAsync(S.d_pairs, 0, sizeof(unsigned long long), S.s));
-  WCSPH_CUDA(cudaMemsetAsync(S.d_counters + 4, 0, sizeof(int), S.s));
-  k_step_begin<<<nblk(std::max<int>(1, (int)S.inst.size())), kBlock, 0, S.s>>>(a);
+  a.zero_pairs = 1;
+  k_step_begin<<<1, kBlock, 0, S.s>>>(a);
   if (n > 0) {
     k_kick_refresh<<<nblk(n), kBlock, 0, S.s>>>(a, 0, 0);
     if (density_pass) {

@@ -125,6 +125,8 @@ struct StepArgs {
   int n_host;             // particle slots in use (upper bound of live)
   int n_inst;
   unsigned long long* pair_count;
+  long long cells;        // cells of all instances (cell_start, cell_end)
+  int zero_pairs;         // the step's begin clears pair_count
   int* run_list;          // linear index of every non-empty cell (unordered)
   int* run_count;         // number of entries in run_list
   int init_filter;        // initial-pass Shepard filter launch (main.cpp:75)
@@ -180,35 +182,49 @@ __device__ __forceinline__ int density_kind(const StepArgs& a, const InstParams&
 }
 
 // ------------------------------------------------------------ step begin
-// One thread per instance: rotate dt, advance time, mark finished.
-__global__ void k_step_begin(StepArgs a) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < a.n_inst) {
-    InstDyn& d = a.dyn[k];
-    const InstParams& P = a.params[k];
-    const int ph = a.phase[k];
-    if (!a.list_reuse) {  // the binning sets them again; a list step keeps the build's order
-      d.range_lo = 0x7fffffff;
-      d.range_hi = 0;
-    }
-    if (ph == PH_STEP && P.active) {
-      const float dt = d.finished ? 0.0f : bits_f(d.dt_next_bits);
-      d.dt_cur = dt;
-      d.dt_next_bits = 0x7f800000u;  // +inf
-      if (dt > 0.0f) {
-        d.time += (double)dt;
-        d.steps += 1;
-        if (P.t_end > 0.0 && d.time >= P.t_end) d.finished = 1;
-      }
-    } else if (ph == PH_INIT) {
-      d.dt_cur = 0.0f;
-      d.dt_next_bits = 0x7f800000u;
-    } else {
-      d.dt_cur = 0.0f;
-    }
-    if (a.dens_any && (ph == PH_INIT || ph == PH_PROBE || density_kind(a, P, d, ph))) atomicOr(a.dens_any, 1);
+// Instance k's part: rotate dt, advance time, mark finished.
+__device__ __forceinline__ void begin_instance(const StepArgs& a, int k) {
+  InstDyn& d = a.dyn[k];
+  const InstParams& P = a.params[k];
+  const int ph = a.phase[k];
+  if (!a.list_reuse) {  // the binning sets them again; a list step keeps the build's order
+    d.range_lo = 0x7fffffff;
+    d.range_hi = 0;
   }
-  if (k == 0 && !a.list_reuse) *a.n_alive = a.n_host;
+  if (ph == PH_STEP && P.active) {
+    const float dt = d.finished ? 0.0f : bits_f(d.dt_next_bits);
+    d.dt_cur = dt;
+    d.dt_next_bits = 0x7f800000u;  // +inf
+    if (dt > 0.0f) {
+      d.time += (double)dt;
+      d.steps += 1;
+      if (P.t_end > 0.0 && d.time >= P.t_end) d.finished = 1;
+    }
+  } else if (ph == PH_INIT) {
+    d.dt_cur = 0.0f;
+    d.dt_next_bits = 0x7f800000u;
+  } else {
+    d.dt_cur = 0.0f;
+  }
+  if (a.dens_any && (ph == PH_INIT || ph == PH_PROBE || density_kind(a, P, d, ph))) atomicOr(a.dens_any, 1);
+}
+
+// What a pass counts up from zero; before begin_instance, with a barrier between.
+__device__ __forceinline__ void begin_counters(const StepArgs& a) {
+  if (a.dens_any) *a.dens_any = 0;
+  if (a.zero_pairs) *a.pair_count = 0ull;
+  if (!a.list_reuse) {
+    *a.n_alive = a.n_host;
+    *a.run_count = 0;
+  }
+}
+
+// One block: the counters, then every instance.  (A kernel of the step graph
+// costs 3 to 4 us however little it does, a memset node 2.)
+__global__ void k_step_begin(StepArgs a) {
+  if (threadIdx.x == 0) begin_counters(a);
+  __syncthreads();
+  for (int k = threadIdx.x; k < a.n_inst; k += blockDim.x) begin_instance(a, k);
 }
 
 // ------------------------------------------------------- kick + binning
@@ -267,6 +283,8 @@ __device__ __forceinline__ bool kick_particle(const StepArgs& a, const InstParam
 // step builds in full.
 __global__ void k_kick_bin(StepArgs a) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  // the empty cell table that k_permute fills
+  for (long long c = p; c < a.cells; c += (long long)gridDim.x * blockDim.x) a.cell_start[c] = 0, a.cell_end[c] = 0;
   if (p >= a.n_host) return;
   uint32_t f = a.main.flags[p];
   const int inst = f & kInstMask;
@@ -558,16 +576,13 @@ __device__ __forceinline__ void copy_state(const StepArgs& a, int p) {
   a.main.flags[p] = a.alt.flags[p];
 }
 
-// Dead tail [n_alive, n_host): carry the slots over to main unchanged so that
-// removed particles keep their last state until the host compacts.
-__global__ void k_copy_dead(StepArgs a) {
-  const int p = *a.n_alive + blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= a.n_host) return;
-  a.main.pos[p] = a.alt.pos[p];
-  a.main.vel[p] = a.alt.vel[p];
-  a.main.acc[p] = a.alt.acc[p];
-  a.main.pid[p] = a.alt.pid[p];
-  a.main.flags[p] = a.alt.flags[p];
+// Dead tail [n_alive, n_host): the hydro pass of a binning pass carries the
+// slots over to main unchanged so that removed particles keep their last state
+// until the host compacts.  Called by every thread of a grid.
+__device__ __forceinline__ void copy_dead(const StepArgs& a) {
+  for (int p = *a.n_alive + (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; p < a.n_host;
+       p += gridDim.x * gridDim.y * blockDim.x)
+    copy_state(a, p);
 }
 
 // Initial Shepard filter of main.cpp:75 (after the initial hydro pass).

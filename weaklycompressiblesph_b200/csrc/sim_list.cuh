@@ -86,7 +86,8 @@ __device__ __forceinline__ float velocity_quantum(float vb, float c0) {
   return __uint_as_float(((__float_as_uint(v) >> 23) + 1u - 15u) << 23);
 }
 
-// One thread, after k_step_begin: the step's build decision, the counters,
+// One block begins a list-mode step: k_step_begin's work (keeping the build's
+// order), then the step's build decision, the counters,
 // and (in a graph) the condition of the node that selects the build or the
 // list-step branch.  An instance needs new lists when the largest
 // displacement its particles can reach in this step, d + dt s + dt^2/2 acc
@@ -100,9 +101,15 @@ __device__ __forceinline__ float velocity_quantum(float vb, float c0) {
 // records the same motion bounds this step's velocities, s + dt acc, which
 // sets the instance's velocity quantum (kept when there is no motion yet).
 __global__ void k_list_set(StepArgs a, int interval, cudaGraphConditionalHandle cond, int use_cond) {
+  __shared__ int need, live, keeps;
   unsigned* lf = a.list_flags;
-  int need = 0, live = 0;
-  for (int k = 0; k < a.n_inst; ++k) {
+  if (threadIdx.x == 0) {
+    begin_counters(a);
+    need = live = 0;
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < a.n_inst; k += blockDim.x) {
+    begin_instance(a, k);
     const InstParams& P = a.params[k];
     const float dt = a.dyn[k].dt_cur;
     unsigned* w = a.inst_motion + 3 * k;
@@ -117,36 +124,41 @@ __global__ void k_list_set(StepArgs a, int interval, cudaGraphConditionalHandle 
       }
     }
     if (P.active) {
-      ++live;
-      need += moved;
+      atomicAdd(&live, 1);
+      if (moved) atomicAdd(&need, 1);
     }
     a.inst_keep[k] = moved ? 0 : (near ? 2 : 1);  // read only in a partial build (2: joins one)
     w[0] = w[1] = w[2] = 0u;  // refilled by this step's list pass
   }
-  const bool overflowed = lf[kLfOverflowPending] != 0u;
-  const bool full = lf[kLfForce] != 0u || overflowed || (int)lf[kLfSince] >= interval || lf[kLfDeaths] != 0u ||
-                    (need > 0 && need == live);
-  const bool build = full || need > 0;
-  if (overflowed) ++lf[kLfOverflows];
-  if (build) {
-    ++lf[kLfBuilds];
-    lf[kLfForce] = 0u;
-    lf[kLfOverflowPending] = 0u;
-  } else {
-    ++lf[kLfListSteps];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const bool overflowed = lf[kLfOverflowPending] != 0u;
+    const bool full = lf[kLfForce] != 0u || overflowed || (int)lf[kLfSince] >= interval || lf[kLfDeaths] != 0u ||
+                      (need > 0 && need == live);
+    const bool build = full || need > 0;
+    if (overflowed) ++lf[kLfOverflows];
+    if (build) {
+      ++lf[kLfBuilds];
+      lf[kLfForce] = 0u;
+      lf[kLfOverflowPending] = 0u;
+    } else {
+      ++lf[kLfListSteps];
+    }
+    if (full) {
+      lf[kLfSince] = 1u;
+      lf[kLfDeaths] = 0u;
+    } else {
+      ++lf[kLfSince];
+    }
+    if (build && !full) ++lf[kLfPartials];
+    lf[kLfPartial] = (build && !full) ? 1u : 0u;
+    lf[kLfDecision] = build ? 1u : 0u;
+    keeps = build && !full;
+    if (use_cond) cudaGraphSetConditional(cond, build ? 1u : 0u);
   }
-  if (full) {
-    lf[kLfSince] = 1u;
-    lf[kLfDeaths] = 0u;
-  } else {
-    ++lf[kLfSince];
-  }
-  if (build && !full) ++lf[kLfPartials];
-  for (int k = 0; k < a.n_inst; ++k)  // only a partial build keeps lists, and the instances near the bound join it
-    a.inst_keep[k] = (!build || full || a.inst_keep[k] == 2) ? 0 : a.inst_keep[k];
-  lf[kLfPartial] = (build && !full) ? 1u : 0u;
-  lf[kLfDecision] = build ? 1u : 0u;
-  if (use_cond) cudaGraphSetConditional(cond, build ? 1u : 0u);
+  __syncthreads();
+  for (int k = threadIdx.x; k < a.n_inst; k += blockDim.x)  // only a partial build keeps lists, and the instances near the bound join it
+    a.inst_keep[k] = (!keeps || a.inst_keep[k] == 2) ? 0 : a.inst_keep[k];
 }
 
 // A list step's kick (kick_particle, no wrapping), in place in the build's
@@ -491,7 +503,7 @@ __device__ __forceinline__ void h16_pair2(const StepArgs& a, const InstParams& P
 }
 
 // The list pass over particle slots below the build's live count (the
-// particles of the build's cell table; the dead tail is k_copy_dead's), on
+// particles of the build's cell table; the dead tail is only carried over), on
 // list steps and right after the scan of a build step: TPI threads per
 // particle walk its list row, each taking every TPI-th group of four entries
 // (one 16-byte load), and sum two entries at a time in the f32x2 halves of
@@ -622,6 +634,8 @@ __device__ __forceinline__ void hydro_list_body(const StepArgs& a) {
       sv = fmaxf(vsa, vsb);
       scnt = ca + cb;
     }
+  } else if (p < a.n_host && sub == 0 && a.alt.pos != a.main.pos) {
+    copy_state(a, p);  // the dead tail of a build (list steps leave it in place)
   }
 #pragma unroll
   for (int o = 1; o < TPI; o <<= 1) {  // every lane takes part; a particle's TPI lanes are adjacent

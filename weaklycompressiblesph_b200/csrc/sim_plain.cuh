@@ -297,6 +297,7 @@ __device__ __forceinline__ void cell_pass(const StepArgs& a, PlainTile<PASS>& S)
 __global__ void __launch_bounds__(32, 12) k_hydro_plain(const __grid_constant__ StepArgs a) {
   __shared__ PlainTile<PLAIN_HYDRO> S;
   cell_pass<PLAIN_HYDRO>(a, S);
+  copy_dead(a);
 }
 
 // Summation rho_i = m sum_j W_ij (self included) or the Shepard filter of

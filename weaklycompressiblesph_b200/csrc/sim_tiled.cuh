@@ -428,6 +428,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_hydro_tiled(StepArgs a) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(full, pairs, o);
   if (lane == 0 && pairs) atomicAdd(a.pair_count, pairs);
+  copy_dead(a);
 }
 
 struct TiledLaunch {
