@@ -7,9 +7,9 @@
 // caller's arrays, packed as the caller holds them, into buffers that are free
 // between passes.  They then cross the link piece by piece into a ring of
 // blocks, each copied out by a few host threads while the next ones are
-// in flight.  1.25 M particles (56 MB): 70 -> 6.6 ms, 65,000: 1.43 -> 0.34 ms;
-// a probe of 1.25 M 35 -> 5.6 ms.  Bound by the host's first
-// touch of the caller's arrays.
+// in flight.  1.25 M particles (56 MB): 70 -> 6.7 ms, 65,000: 1.43 -> 0.4, 12,600: 0.36 -> 0.12;
+// a probe of 1.25 M 35 -> 6 ms.  Bound by the host's first touch of the caller's
+// arrays.
 #pragma once
 #include <omp.h>
 #include <sys/mman.h>
@@ -89,13 +89,12 @@ struct ReadField {
 };
 
 // Ring of host blocks the pieces of a read pass through, allocated by the
-// first read for the largest one the solver can have, at most kBlockBytes each,
-// and given back with the solver.  Blocks from kPinBytes on are huge pages
-// registered with the device: 12 MB cost 0.8 ms that way and 5.6 ms from
-// cudaMallocHost.  Below, pinning (0.4 ms) would cost a solver's first read more
-// than the copies of several hundred reads gain by it (64 KB: 12 against 17 us),
-// and where it fails ordinary memory serves as well: copies into it are
-// synchronous.
+// first read for the largest one the solver can have, at most kBlockBytes each
+// (1.6 M particles, 72 MB: 4.6 ms with blocks of 8 MB, 7.3 with 4), and given
+// back with the solver.  Blocks from kPinBytes on are huge pages registered with
+// the device: 12 MB cost 0.8 ms that way and 5.6 ms from cudaMallocHost.  Below,
+// and where it fails, ordinary memory serves; copies into it are synchronous
+// (12,600 particles: 0.22 ms a read, 0.10 registered).
 class ReadRing {
  public:
   ~ReadRing() { release(); }
@@ -109,8 +108,11 @@ class ReadRing {
       int field, i0, i1;  // field -1: cover
       size_t off;
     };
-    // 45 bytes a particle and the alignment of a handful of pieces
-    if (int rc = reserve((size_t)std::min<long long>(kBlockBytes, (48 * n_max + 8191) / 4096 * 4096))) return rc;
+    // 45 bytes a particle and the alignment of a handful of pieces: a quarter of
+    // that a block, but 1 MB in one
+    const long long whole = 48 * n_max + 4096;
+    const long long block = std::min<long long>(kBlockBytes, std::max<long long>(whole / 4, std::min<long long>(whole, 1 << 20)));
+    if (int rc = reserve((size_t)(block + 4095) / 4096 * 4096)) return rc;
     // Pieces in order, cut into batches of one block each.
     std::vector<std::vector<Piece>> batch(1);
     size_t used = kHead;  // the first block starts with the count of missing particles
@@ -204,9 +206,9 @@ class ReadRing {
   }
 
  private:
-  static constexpr size_t kBlocks = 3, kBlockBytes = 4 << 20, kPinBytes = 1 << 20, kHead = 16;
+  static constexpr size_t kBlocks = 3, kBlockBytes = 8 << 20, kPinBytes = 128 << 10, kHead = 16;
   static constexpr size_t kSlice = 128 << 10;  // bytes of a host thread's share, at least
-  static constexpr int kThreads = 16;
+  static constexpr int kThreads = 10;  // 309,000 particles: 0.8 ms, with 16 threads 1.3 (they share the cores with the caller)
 
   template <class Body>
   static void slices(int i0, int i1, size_t el, Body&& body) {
