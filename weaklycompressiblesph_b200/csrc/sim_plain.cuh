@@ -39,37 +39,43 @@ struct alignas(16) PlainTile {
   uint32_t mask[kScanTile / 32][32];
 };
 
-struct PairConst {
-  float h, eh2, Kg, iH, alpha, beta, nu4;
+// Operands of pair_terms for the lane's particle and its instance: packed
+// duplicates (the factors carry signs, which are exact).
+struct PlainI {
+  f2 X, Y, Z, VX, VY, VZ, RHO, PO, CI;
+  f2 NIH, NKG, EH2, H, BETA, NAH, NNU4;  // -1/2h, -Kg, eps h^2, h, beta, -alpha/2, -4 nu
 };
-struct PairTerm {
-  float x, y, z, g, drdv, mu;
+// The terms of two pairs, one per half (force.h:38-57 for uniform h, m, nu): NG
+// is minus the gradient factor.  Every product, sum and fma is the one that the
+// scalar expression (visc * dvx - pg * dx and so on) is compiled to, so that the
+// terms are those of a scalar loop to the bit.
+struct PairTerms {
+  f2 R2, X, Y, Z, NG, DRDV, MU;
 };
-// Terms of the pair of particle (I, IB, ci) with candidate u; false for the
-// particle itself, and any at its very place.
-__device__ __forceinline__ bool pair_term(const PairConst& C, const float4& I, const float4& IB, float ci, int u,
-                                          const PlainTile<PLAIN_HYDRO>& S, PairTerm& t) {
-  const float dx = __fsub_rn(I.x, S.pos[0][u]), dy = __fsub_rn(I.y, S.pos[1][u]), dz = __fsub_rn(I.z, S.pos[2][u]);
-  const float r2 = dist2(dx, dy, dz);
-  const float4 JB = S.b[u];
-  const float2 pc = S.pc[u];
-  const float rinv = rsqrtf(r2);
-  const float g = spline_F(r2 * rinv * C.iH) * C.Kg * rinv;
-  const float dvx = IB.x - JB.x, dvy = IB.y - JB.y, dvz = IB.z - JB.z;
-  const float drdv = dx * dvx + dy * dvy + dz * dvz;
-  const float rden = __frcp_rn(r2 + C.eh2);
-  const float mu = drdv < 0.0f ? C.h * drdv * rden : 0.0f;
-  const float rs = __frcp_rn(IB.w + JB.w);
-  const float av = (C.beta * mu - C.alpha * 0.5f * (ci + pc.y)) * mu * 2.0f * rs;
-  const float pg = (I.w + pc.x + av) * g;
-  const float visc = C.nu4 * g * r2 * rs * rden;
-  t.x = visc * dvx - pg * dx;
-  t.y = visc * dvy - pg * dy;
-  t.z = visc * dvz - pg * dz;
-  t.g = g;
-  t.drdv = drdv;
-  t.mu = mu;
-  return r2 > 0.0f;
+__device__ __forceinline__ PairTerms pair_terms(const PlainI& I, const PlainTile<PLAIN_HYDRO>& S, int u0, int u1) {
+  PairTerms t;
+  const f2 DX = sub2(I.X, pk(S.pos[0][u0], S.pos[0][u1])), DY = sub2(I.Y, pk(S.pos[1][u0], S.pos[1][u1])),
+           DZ = sub2(I.Z, pk(S.pos[2][u0], S.pos[2][u1]));
+  t.R2 = fma2(DZ, DZ, fma2(DY, DY, mul2(DX, DX)));  // == dist2 per half
+  const float4 B0 = S.b[u0], B1 = S.b[u1];
+  const float2 p0 = S.pc[u0], p1 = S.pc[u1];
+  const f2 RINV = rsqrt2(t.R2), Q = mul2(t.R2, RINV);
+  const f2 A = max0_2(fma2(Q, I.NIH, dup(1.0f))), B = max0_2(fma2(Q, I.NIH, dup(0.5f)));
+  const f2 F = fma2(mul2(dup(12.0f), B), B, mul2(mul2(dup(-3.0f), A), A));
+  t.NG = mul2(mul2(F, I.NKG), RINV);
+  const f2 DVX = sub2(I.VX, pk(B0.x, B1.x)), DVY = sub2(I.VY, pk(B0.y, B1.y)), DVZ = sub2(I.VZ, pk(B0.z, B1.z));
+  t.DRDV = fma2(DZ, DVZ, fma2(DX, DVX, mul2(DY, DVY)));
+  const f2 D = add2(t.R2, I.EH2), R = add2(I.RHO, pk(B0.w, B1.w));
+  const f2 RDEN = pk(__frcp_rn(lo(D)), __frcp_rn(hi(D))), RS = pk(__frcp_rn(lo(R)), __frcp_rn(hi(R)));
+  const f2 MUr = mul2(mul2(I.H, t.DRDV), RDEN);
+  t.MU = pk(lo(t.DRDV) < 0.0f ? lo(MUr) : 0.0f, hi(t.DRDV) < 0.0f ? hi(MUr) : 0.0f);
+  const f2 AV = mul2(mul2(fma2(I.BETA, t.MU, mul2(I.NAH, add2(I.CI, pk(p0.y, p1.y)))), t.MU), dup(2.0f));
+  const f2 NPG = mul2(fma2(AV, RS, add2(I.PO, pk(p0.x, p1.x))), t.NG);
+  const f2 VISC = mul2(mul2(mul2(mul2(I.NNU4, t.NG), t.R2), RS), RDEN);
+  t.X = fma2(VISC, DVX, mul2(NPG, DX));
+  t.Y = fma2(VISC, DVY, mul2(NPG, DY));
+  t.Z = fma2(VISC, DVZ, mul2(NPG, DZ));
+  return t;
 }
 __device__ __forceinline__ bool density_term(const float4& I, int u, const PlainTile<PLAIN_DENSITY>& S, float iH,
                                              float& w) {
@@ -140,7 +146,6 @@ __device__ __forceinline__ void cell_pass(const StepArgs& a, PlainTile<PASS>& S)
     const int delta = start - first;
     const float H2 = P.H2, cull = H2 * kCullMargin, iH = P.inv_H;
     const f2 NH2 = dup(-H2);
-    const PairConst C{P.h, P.eh2, P.Kg, iH, P.alpha, P.beta, P.nu4};
     const int vs = P.vsig_mode;
     const bool shep = kind == 2;
 
@@ -160,7 +165,14 @@ __device__ __forceinline__ void cell_pass(const StepArgs& a, PlainTile<PASS>& S)
       const float bz0 = warp_min_f(mine ? I.z : big), bz1 = warp_max_f(mine ? I.z : -big);
       const f2 IX = dup(I.x), IY = dup(I.y), IZ = dup(I.z);
       const float rho_i = IB.w;
-      float ax = 0.f, ay = 0.f, az = 0.f, dsum = 0.f, vsig = 0.f;
+      PlainI i2;
+      if (PASS == PLAIN_HYDRO) {
+        i2.X = IX, i2.Y = IY, i2.Z = IZ, i2.VX = dup(IB.x), i2.VY = dup(IB.y), i2.VZ = dup(IB.z);
+        i2.RHO = dup(IB.w), i2.PO = dup(I.w), i2.CI = dup(ci);
+        i2.NIH = dup(-iH), i2.NKG = dup(-P.Kg), i2.EH2 = dup(P.eh2), i2.H = dup(P.h);
+        i2.BETA = dup(P.beta), i2.NAH = dup(-(P.alpha * 0.5f)), i2.NNU4 = dup(-P.nu4);
+      }
+      float ax = 0.f, ay = 0.f, az = 0.f, ndsum = -0.f, vsig = 0.f;
       float sum = 0.5f, one = 0.5f / rho_i;  // self term: w(0) = 1/2
       unsigned cnt = 0;
 
@@ -248,19 +260,18 @@ __device__ __forceinline__ void cell_pass(const StepArgs& a, PlainTile<PASS>& S)
               if (shep) one += w1 / S.rho[u1];
             }
           } else {
-            PairTerm t0, t1;
-            const bool b0 = pair_term(C, I, IB, ci, u0, S, t0), b1 = u1 >= 0 && pair_term(C, I, IB, ci, u1, S, t1);
-            if (b0) {
+            const PairTerms t = pair_terms(i2, S, u0, max(u1, 0));
+            if (lo(t.R2) > 0.0f) {  // not the particle itself, nor any at its very place
               ++cnt;
-              ax += t0.x, ay += t0.y, az += t0.z;
-              dsum += t0.g * t0.drdv;
-              vsig = fmaxf(vsig, vs ? -t0.mu : t0.mu);
+              ax += lo(t.X), ay += lo(t.Y), az += lo(t.Z);
+              ndsum = __fmaf_rn(lo(t.NG), lo(t.DRDV), ndsum);
+              vsig = fmaxf(vsig, vs ? -lo(t.MU) : lo(t.MU));
             }
-            if (b1) {
+            if (u1 >= 0 && hi(t.R2) > 0.0f) {
               ++cnt;
-              ax += t1.x, ay += t1.y, az += t1.z;
-              dsum += t1.g * t1.drdv;
-              vsig = fmaxf(vsig, vs ? -t1.mu : t1.mu);
+              ax += hi(t.X), ay += hi(t.Y), az += hi(t.Z);
+              ndsum = __fmaf_rn(hi(t.NG), hi(t.DRDV), ndsum);
+              vsig = fmaxf(vsig, vs ? -hi(t.MU) : hi(t.MU));
             }
           }
         }
@@ -273,7 +284,7 @@ __device__ __forceinline__ void cell_pass(const StepArgs& a, PlainTile<PASS>& S)
         bool dt_valid = false;
         if (mine) {
           const uint32_t f = a.alt.flags[p];
-          finish_hydro(a, p, P, inst, ph, f, ax, ay, az, dsum, vsig, cnt, dt_cand, dt_valid);
+          finish_hydro(a, p, P, inst, ph, f, ax, ay, az, -ndsum, vsig, cnt, dt_cand, dt_valid);
           if (!(f & kGhostBit)) pairs += cnt;  // pairs are counted for owned particles only
         }
         dt_min(a.dyn, inst, dt_cand, dt_valid);
