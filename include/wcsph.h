@@ -167,7 +167,7 @@ int wcsph_filter_retrieve(int32_t tag, int32_t n_walk, const int32_t* n_i, void*
 /* ------------------------------------------------------------------------- */
 
 typedef enum {
-  WCSPH_PREC_FP32 = 0,  /* plain FP32 pair arithmetic, one thread per i-particle          */
+  WCSPH_PREC_FP32 = 0,  /* plain FP32 pair arithmetic, sums in the order of the search    */
   WCSPH_PREC_TILED = 1, /* FP32, shared-memory j-tiles, ballot-compacted pair queues      */
   WCSPH_PREC_HALF2 = 2  /* with neighbour lists: the list pass gathers 16-byte compact
                            j-records (16-bit cell-relative positions and velocities, FP32

@@ -3,9 +3,8 @@
 //
 // Step (one CUDA graph, main.cpp:89-133 order):
 //   k_step_begin   dt rotation (integral.h:2-12 result of the previous pass), time += dt
-//   k_kick_bin     initialKick + fullDrift + predict (class.h:146-159), Morton cell key
+//   k_kick_bin     initialKick + fullDrift + predict (class.h:146-159), Morton cell key, empty cell table
 //   radix sort     (keys, slot) pairs, stable
-//   memset x2      cell table
 //   k_permute      gather main -> alt in sorted order, cell table, EoS j-records
 //   k_density/eos  density pass when an instance wants one this step
 //   k_hydro        pair sums, gravity, finalKick, density floor, next dt
@@ -231,6 +230,9 @@ static void mark_drained(SimImpl& S) {
 }
 
 constexpr int kBlock = 256;
+constexpr int kClearBlocks = 1184;  // enough to clear cells at the memory's rate
+// Threads of the one block that begins a step.
+static int begin_threads(const SimImpl& S) { return S.inst.size() <= 256 ? 256 : 1024; }
 static inline int nblk(long long n) { return (int)std::max<long long>(1, (n + kBlock - 1) / kBlock); }
 
 // Enqueue one pass of the pipeline.  init_filter adds the initial Shepard
@@ -260,11 +262,12 @@ static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, 
     k_begin_build<<<nblk(std::max<int>(1, (int)S.inst.size())), kBlock, 0, S.s>>>(a);
   } else {
     if (ev) WCSPH_CUDA(cudaEventRecord(ev[0], S.s));
-    k_step_begin<<<1, kBlock, 0, S.s>>>(a);
+    k_step_begin<<<1, begin_threads(S), 0, S.s>>>(a);
   }
   ++L;
   if (n > 0) {
-    k_kick_bin<<<nblk(n), kBlock, 0, S.s>>>(a);
+    // blocks beyond the particles' clear the cell table of a sparse domain
+    k_kick_bin<<<std::max(nblk(n), std::min(nblk(S.total_cells), kClearBlocks)), kBlock, 0, S.s>>>(a);
     ++L;
     size_t bytes = S.cub_bytes;
     WCSPH_CUDA(cub::DeviceRadixSort::SortPairs(S.cub_tmp, bytes, S.keys_in, S.keys_out, S.vals_in, S.vals_out, n, 0,
@@ -613,7 +616,7 @@ static int enqueue_list_prologue(SimImpl& S, const StepArgs& a0, cudaGraphCondit
   a.x0 = S.x0;
   if (ev) WCSPH_CUDA(cudaEventRecord(ev[0], S.s));
   a.zero_pairs = 1;
-  k_list_set<<<1, kBlock, 0, S.s>>>(a, S.opt.list_interval, cond, use_cond ? 1 : 0);
+  k_list_set<<<1, begin_threads(S), 0, S.s>>>(a, S.opt.list_interval, cond, use_cond ? 1 : 0);
   WCSPH_CUDA(cudaGetLastError());
   return 0;
 }
@@ -652,7 +655,7 @@ static int list_step(SimImpl& S, bool graph, cudaEvent_t* ev, bool* built = null
 }
 
 // The list-mode step graph: the prologue, then a conditional node whose IF
-// branch is a build step (binning, sort, scan-only tiled pass, list pass) and
+// branch is a build step (binning, sort, list scan, list pass) and
 // whose ELSE branch is a list step (kick and refresh in place, list passes),
 // then the copy of the flags to the host.
 static int capture_list_graph(SimImpl& S) {
@@ -1527,7 +1530,7 @@ static int enqueue_probe_lists(SimImpl& S, int density_pass) {
   a.alt = a.main;
   const int n = S.n_host;
   a.zero_pairs = 1;
-  k_step_begin<<<1, kBlock, 0, S.s>>>(a);
+  k_step_begin<<<1, begin_threads(S), 0, S.s>>>(a);
   if (n > 0) {
     k_kick_refresh<<<nblk(n), kBlock, 0, S.s>>>(a, 0, 0);
     if (density_pass) {

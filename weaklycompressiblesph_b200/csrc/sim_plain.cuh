@@ -3,22 +3,24 @@
 // search (for_each_neighbor), summed one after the other by the particle's lane.
 //
 // One warp per non-empty cell, up to 32 of its particles at a time.  The
-// candidates of the 27 neighbour cells are staged in shared memory with all
-// that a pair needs, runs of slots along x at a time, when they lie within the
-// support radius of the batch's bounding box; every lane tests 32 of them at a
-// time into a bit mask (packed f32x2, the sign of r^2 - H^2), and evaluates the
-// pairs of its masks.  The additions and their order are those of a loop over
-// every candidate, so that the block shape and the staging never change a bit.
+// candidates of the 27 neighbour cells are staged in shared memory with all that
+// a pair needs when they lie within the support radius of the batch's bounding
+// box; every lane tests 32 of them at a time into a bit mask (packed f32x2, the
+// sign of r^2 - H^2), and evaluates the pairs of its masks.  The additions and
+// their order are those of a loop over every candidate, so that the block shape
+// and the staging never change a bit.
 //
 // Against one thread per particle that walked the 27 cells itself, a step's
-// hydro pass: dam break of 12,600 particles 163 -> 41 us, of 54,500 186 -> 80,
-// of 477,000 559 -> 523, of 1.25 M 1395 -> 1356; cells of 83 particles (8,100 in
-// all) 492 -> 370.  Density pass of a lattice of 64,000: 149 -> 81 us.
+// hydro pass: dam break of 12,600 particles 163 -> 39 us, of 54,500 186 -> 76,
+// of 477,000 559 -> 468, of 1.25 M 1395 -> 1250; cells of 83 particles (8,100 in
+// all) 492 -> 340.  Density pass of a lattice of 64,000: 149 -> 81 us.
 // Small solvers are bound by the instructions of one cell's warp (9,000, at six
-// cycles each), large ones by the same stream at 12 warps an SM.  Two candidates'
-// terms are evaluated side by side: one at a time is 570 us at 477,000.  Four
-// warps a batch that rank the candidates and share the terms through shared
-// memory are no faster for small solvers (41 us) and slower for large (943 us).
+// cycles each), large ones by the same stream at 14 warps an SM.  Two candidates'
+// terms are evaluated side by side in packed arithmetic (477,000 particles: one
+// at a time 570 us, two scalar streams 523, packed 492, before the tile was cut
+// to 384).  Four warps a batch that rank the candidates and share the terms
+// through shared memory are no faster for small solvers and slower for large
+// (943 us).
 #pragma once
 #include "sim_scan.cuh"
 
@@ -27,16 +29,17 @@ namespace wcsph {
 enum PlainPass { PLAIN_HYDRO, PLAIN_DENSITY };
 
 constexpr int kBatches = 2;  // blocks that share a cell's batches (hydro pass; most density launches have nothing to do)
-constexpr int kStage = 4;  // groups of 32 candidates whose loads are in flight together
+constexpr int kPlainTile = 384;  // candidates (hydro pass, 477,000 particles: 468 us; 448: 504; 320: 440, but lattices lose)
+constexpr int kStage = 2;  // groups of 32 candidates whose loads are in flight together
 
-// Shared memory of a warp: 448 candidates (most cells' in one tile).
+// Shared memory of a warp.
 template <int PASS>
 struct alignas(16) PlainTile {
-  float pos[3][kScanTile];                                // shifted by the periodic image
-  float4 b[PASS == PLAIN_HYDRO ? kScanTile : 1];          // v, rho
-  float2 pc[PASS == PLAIN_HYDRO ? kScanTile : 1];         // P / rho^2, c
-  float rho[PASS == PLAIN_DENSITY ? kScanTile : 1];
-  uint32_t mask[kScanTile / 32][32];
+  float pos[3][kPlainTile];                                // shifted by the periodic image
+  float4 b[PASS == PLAIN_HYDRO ? kPlainTile : 1];          // v, rho
+  float2 pc[PASS == PLAIN_HYDRO ? kPlainTile : 1];         // P / rho^2, c
+  float rho[PASS == PLAIN_DENSITY ? kPlainTile : 1];
+  uint32_t mask[kPlainTile / 32][32];
 };
 
 // Operands of pair_terms for the lane's particle and its instance: packed
@@ -179,7 +182,7 @@ __device__ __forceinline__ void cell_pass(const StepArgs& a, PlainTile<PASS>& S)
       int k0 = 0;  // candidates staged or culled so far
       do {
         int tn = 0;  // staged candidates
-        for (; k0 < total && tn + 32 * kStage <= kScanTile; k0 += 32 * kStage) {
+        for (; k0 < total && tn + 32 * kStage <= kPlainTile; k0 += 32 * kStage) {
           float4 J[kStage], B[kStage];
           float c[kStage], sx[kStage], sy[kStage], sz[kStage];
 #pragma unroll
@@ -305,7 +308,7 @@ __device__ __forceinline__ void cell_pass(const StepArgs& a, PlainTile<PASS>& S)
 // The epilogue adds gravity (Dam2.h:104-108), does the final kick
 // (class.h:160-163), the density floor (Dam2.h:111), and folds the CFL limits
 // of integral.h:2-12 into the instance's next dt.
-__global__ void __launch_bounds__(32, 12) k_hydro_plain(const __grid_constant__ StepArgs a) {
+__global__ void __launch_bounds__(32, 14) k_hydro_plain(const __grid_constant__ StepArgs a) {
   __shared__ PlainTile<PLAIN_HYDRO> S;
   cell_pass<PLAIN_HYDRO>(a, S);
   copy_dead(a);

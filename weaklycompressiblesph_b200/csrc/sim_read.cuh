@@ -91,10 +91,12 @@ struct ReadField {
 // Ring of host blocks the pieces of a read pass through, allocated by the
 // first read for the largest one the solver can have, at most kBlockBytes each
 // (1.6 M particles, 72 MB: 4.6 ms with blocks of 8 MB, 7.3 with 4), and given
-// back with the solver.  Blocks from kPinBytes on are huge pages registered with
-// the device: 12 MB cost 0.8 ms that way and 5.6 ms from cudaMallocHost.  Below,
-// and where it fails, ordinary memory serves; copies into it are synchronous
-// (12,600 particles: 0.22 ms a read, 0.10 registered).
+// back with the solver.  Blocks above kSecondBytes are huge pages registered with
+// the device at once: 12 MB cost 0.8 ms that way and 5.6 ms from cudaMallocHost.
+// Smaller ones are registered by the second read (0.4 ms: more than one read
+// gains by it; 12,600 particles: 0.22 ms a read, 0.10 registered), and those
+// below kPinBytes never.  Unregistered, and where registering fails, ordinary
+// memory serves; copies into it are synchronous.
 class ReadRing {
  public:
   ~ReadRing() { release(); }
@@ -207,6 +209,7 @@ class ReadRing {
 
  private:
   static constexpr size_t kBlocks = 3, kBlockBytes = 8 << 20, kPinBytes = 128 << 10, kHead = 16;
+  static constexpr size_t kSecondBytes = 1 << 20, kHuge = 2 << 20;
   static constexpr size_t kSlice = 128 << 10;  // bytes of a host thread's share, at least
   static constexpr int kThreads = 10;  // 309,000 particles: 0.8 ms, with 16 threads 1.3 (they share the cores with the caller)
 
@@ -223,27 +226,39 @@ class ReadRing {
   int reserve(size_t bytes) {
     for (cudaEvent_t& e : ev_)
       if (!e) WCSPH_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    if (bytes <= bytes_) return 0;
-    const size_t huge = 2 << 20, all = (bytes * kBlocks + huge - 1) / huge * huge;
-    const bool pin = bytes >= kPinBytes;
-    mem_ = static_cast<char*>(pin ? aligned_alloc(huge, all) : malloc(bytes * kBlocks));
+    if (bytes_) {
+      if (!pinned_ && reads_++ == 0) pin();
+      return 0;
+    }
+    const size_t all = bytes < kPinBytes ? bytes * kBlocks : (bytes * kBlocks + kHuge - 1) / kHuge * kHuge;
+    mem_ = static_cast<char*>(bytes < kPinBytes ? malloc(all) : aligned_alloc(kHuge, all));
     if (!mem_) {
-      set_error("read: %zu bytes of host memory are not to be had", bytes * kBlocks);
+      set_error("read: %zu bytes of host memory are not to be had", all);
       return WCSPH_E_NOMEM;
     }
     bytes_ = bytes;
-    if (pin) {
-      madvise(mem_, all, MADV_HUGEPAGE);
-      slices(0, (int)(all / huge), huge, [&](int i0, int i1) { memset(mem_ + huge * i0, 0, huge * (i1 - i0)); });
-      pinned_ = cudaHostRegister(mem_, all, cudaHostRegisterDefault) == cudaSuccess;
-      if (!pinned_) cudaGetLastError();
+    if (bytes > kSecondBytes) {
+      ++reads_;
+      pin();
     }
     return 0;
+  }
+
+  void pin() {
+    if (bytes_ < kPinBytes) return;
+    const size_t all = (bytes_ * kBlocks + kHuge - 1) / kHuge * kHuge;
+    if (bytes_ > kSecondBytes) {
+      madvise(mem_, all, MADV_HUGEPAGE);
+      slices(0, (int)(all / kHuge), kHuge, [&](int i0, int i1) { memset(mem_ + kHuge * i0, 0, kHuge * (i1 - i0)); });
+    }
+    pinned_ = cudaHostRegister(mem_, bytes_ > kSecondBytes ? all : bytes_ * kBlocks, cudaHostRegisterDefault) == cudaSuccess;
+    if (!pinned_) cudaGetLastError();
   }
 
   char* mem_ = nullptr;
   cudaEvent_t ev_[kBlocks] = {};
   size_t bytes_ = 0;  // per block; the same in every read of a solver
+  int reads_ = 0;     // since the blocks were allocated, until they are registered
   bool pinned_ = false;
 };
 
