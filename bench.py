@@ -629,7 +629,8 @@ def main():
                "walks": e["n_walk"], "pair_evaluations_per_pass": e["evaluated"],
                "ms_per_pass": 1e3 * e["s_per_pass"], "dispatch_ms": e["dispatch_ms"], "retrieve_ms": e["retrieve_ms"],
                "pieces_compact": f"{e['pieces_compact']} of {e['pieces']}"}
-        if not args.no_cpu:
+        import oracle
+        if not args.no_cpu and oracle.ref_available():  # without the reference's build there is no CPU figure
             v, desc, cores, _ = cpu_reference(case, e["walks"], e["epi"], e["epj"], args.cpu_seconds,
                                               dev["pairs_per_step"])
             cpu = {"value": v, "unit": UNIT, "cores": cores, "kind": "reference", "sample": desc}
