@@ -1,0 +1,57 @@
+"""Lists that a probe builds, and probes of instances that a build's step did
+not advance: the rows of every active instance are written, whatever its phase.
+
+Counts and forces against the FP64 oracle at the tolerances of the other list
+tests (counts exact; 1e-5 FP32, 1e-3 half2)."""
+import numpy as np
+import pytest
+
+from tests.helpers import small_dam
+from tests.test_lists_gpu import LIST_TOL, oracle_list_check
+from weaklycompressiblesph_b200 import _native as N
+from weaklycompressiblesph_b200.sim import Solver
+
+pytestmark = pytest.mark.gpu
+PRECS = pytest.mark.parametrize("prec", [N.PREC_TILED, N.PREC_HALF2], ids=["tiled", "half2"])
+
+
+def two_dams():
+    return small_dam(dx=0.05, seed=1, vel_sigma=0.2), small_dam(dx=0.04, seed=2, vel_sigma=0.2, column=(0.3, 0.4, 0.6))
+
+
+def check(oracle_lib, case, st, pr, prec):
+    assert (st["alive"] == 1).all()
+    r = oracle_list_check(oracle_lib, case, st, pr, 0)
+    np.testing.assert_array_equal(pr["nbr"], r["cnt"])
+    assert r["acc"] < LIST_TOL[prec] and r["div_v"] < LIST_TOL[prec], r
+    return r["tot"]
+
+
+@PRECS
+def test_probe_on_stale_lists_builds_every_instance(prec, native, oracle_lib):
+    a, b = two_dams()
+    with Solver(a.n + b.n, max_instances=2, precision=prec, list_interval=20, autotune=False) as s:
+        ka, kb = s.add(a), s.add(b)
+        s.step(3)
+        s.probe(ka)              # a search: the lists are dropped
+        s.probe(ka, lists=True)  # builds them
+        builds = s.list_stats()["builds"]
+        check(oracle_lib, b, s.read(kb), s.probe(kb, lists=True), prec)
+        s.step(2)  # reads the lists of the probe
+        assert s.list_stats()["builds"] == builds
+        pairs, states = s.last_pairs(), [s.read(ka), s.read(kb)]
+        tot = [check(oracle_lib, c, st, s.probe(k, lists=True), prec) for c, st, k in zip((a, b), states, (ka, kb))]
+    assert pairs == sum(tot)
+
+
+@PRECS
+def test_probe_of_a_finished_instance(prec, native, oracle_lib):
+    """An instance past its t_end stays in the lists of the builds that follow."""
+    a, b = two_dams()
+    with Solver(a.n + b.n, max_instances=2, precision=prec, list_interval=2, autotune=False) as s:
+        ka, kb = s.add(a, t_end=1e-9), s.add(b)
+        s.step(7)  # builds at every other step
+        assert s.status(ka)["finished"] and s.status(ka)["steps"] == 1 and s.status(kb)["steps"] == 7
+        assert s.list_stats()["builds"] >= 3
+        for c, k in ((a, ka), (b, kb)):
+            check(oracle_lib, c, s.read(k), s.probe(k, lists=True), prec)

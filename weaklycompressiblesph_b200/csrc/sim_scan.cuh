@@ -82,7 +82,9 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_list_scan(const __gr
     const int inst = a.alt.flags[s] & kInstMask;
     if (partial && a.inst_keep[inst]) continue;  // keeps its lists
     const InstParams& P = a.params[inst];
-    if (!wants_force(P, a.dyn[inst], a.phase[inst])) {
+    // every active instance, idle or finished as it may be in this pass: the sort
+    // has moved its particles, and later probes and steps read its rows
+    if (!P.active) {
       for (int p = s + lane; p < e; p += 32) a.list_cnt[p] = 0;
       continue;
     }
@@ -258,7 +260,8 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_list_scan(const __gr
       if (mine) {
         a.list_cnt[ib + lane] = len;
         if (len > L) {
-          a.list_flags[kLfOverflowPending] = 1u;  // the next step rebuilds
+          // the next step rebuilds (a finished instance's particles never move again)
+          if (a.phase[inst] != PH_STEP || a.dyn[inst].dt_cur > 0.0f) a.list_flags[kLfOverflowPending] = 1u;
         } else {  // pad the row to a whole group of four (list_max is a multiple of four)
           for (int k = len; k < ((len + 3) & ~3); ++k) put(k, a.list_pad);
         }
