@@ -9,6 +9,7 @@ import pytest
 from tests.helpers import small_dam
 from tests.test_lists_gpu import LIST_TOL, oracle_list_check
 from weaklycompressiblesph_b200 import _native as N
+from weaklycompressiblesph_b200 import cases
 from weaklycompressiblesph_b200.sim import Solver
 
 pytestmark = pytest.mark.gpu
@@ -55,3 +56,20 @@ def test_probe_of_a_finished_instance(prec, native, oracle_lib):
         assert s.list_stats()["builds"] >= 3
         for c, k in ((a, ka), (b, kb)):
             check(oracle_lib, c, s.read(k), s.probe(k, lists=True), prec)
+
+
+@pytest.mark.parametrize("density_pass", [1, 2], ids=["summation", "shepard"])
+@PRECS
+def test_probe_of_overflowed_lists(prec, density_pass, native, oracle_lib):
+    """Particles with more neighbours than a list holds (about 500 at h = 2.5
+    dx): the density pass of a probe searches for them as its pair sums do."""
+    case = small_dam(dx=0.05, seed=8, phys=cases.Physics(h_over_dx=2.5))
+    with Solver(case.n, precision=prec, list_interval=10, autotune=False) as s:
+        k = s.add(case)
+        s.step(2)
+        assert s.list_stats()["overflows"] >= 1
+        st = s.read(k)
+        pr = s.probe(k, density_pass=density_pass, lists=True)
+    r = oracle_list_check(oracle_lib, case, st, pr, density_pass)
+    np.testing.assert_array_equal(pr["nbr"], r["cnt"])
+    assert r["dens"] < 1e-5 and r["acc"] < LIST_TOL[prec] and r["div_v"] < LIST_TOL[prec], r

@@ -1535,6 +1535,7 @@ static int enqueue_probe_lists(SimImpl& S, int density_pass) {
     k_kick_refresh<<<nblk(n), kBlock, 0, S.s>>>(a, 0, 0);
     if (density_pass) {
       if (int rc = launch_density_list(a, n, S.s, h16_lists(S.opt))) return rc;
+      k_density_overflow<<<nblk(n), kBlock, 0, S.s>>>(a);  // no particle has moved since a build that overflowed
       k_eos<<<nblk(n), kBlock, 0, S.s>>>(a);
     }
     const bool h16 = S.opt.precision == WCSPH_PREC_HALF2;
