@@ -367,9 +367,10 @@ int32_t wcsph_sim_kernels_per_step(wcsph_sim* sim);
  * from the density instead of gathered (5), or both (6); in the FP32 pass
  * shape 0.  Shapes 0,
  * 2 and 4 sum in one order, 1 and 3 in another; 5 and 6 round P/rho^2
- * differently: results agree to FP32 rounding), out[2] log2 particle bucket
- * it was tuned for (-1:
- * defaults, not tuned), out[3] shape of the list build's scan (0, 3, 5: 4
+ * differently: results agree to FP32 rounding; unless list_shape fixes one, a
+ * tuned solver takes a shape of the order that its present particle count asks
+ * for), out[2] log2 particle bucket it was tuned for (-1: defaults, not tuned),
+ * out[3] shape of the list build's scan (0, 3, 5: 4
  * warps per block, 1: 2, 2, 4, 6: 8; all build the same lists). */
 int wcsph_sim_tuning(wcsph_sim* sim, int32_t* out4);
 /* Neighbour-list counters (list_interval > 0): out[0] list builds, out[1]

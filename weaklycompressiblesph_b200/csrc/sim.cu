@@ -74,7 +74,8 @@ struct SimImpl {
   long long total_cells = 0;
   bool any_density = false;
   int tile_shape = 0;          // tiled pair-kernel shape, chosen by the autotuner
-  int list_shape = 0;          // list-pass launch shape (kListShapes), chosen by the autotuner
+  int list_shape = 0;          // list-pass launch shape (kListShapes), chosen by the autotuner (list_shape_now)
+  int sms = 0;                 // multiprocessors of the device
   int build_shape = 0;         // list build's scan shape (kBuildShapes), chosen by the autotuner
   int tuned_bucket = -1;       // log2 particle bucket of the last tuning
   cudaGraphExec_t gexec = nullptr;
@@ -251,6 +252,16 @@ __global__ void k_begin_build(StepArgs a) {
   }
 }
 
+// The list pass's launch shape at the present size: the fixed one, the default
+// before any tuning, or the tuned one while it sums in the order that
+// list_threads asks for now.  A solver that has grown or shrunk past a line of
+// that rule since it was tuned takes the default shape of the other order.
+static int list_shape_now(const SimImpl& S) {
+  if ((S.opt.list_shape & 0xff) > 0 || S.tuned_bucket < 0) return S.list_shape;
+  const int threads = list_threads(S.n_host, h16_lists(S.opt), S.sms);
+  return kListShapeTPI[S.list_shape] == threads ? S.list_shape : threads == 2 ? 1 : 0;
+}
+
 static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, int* launches,
                         cudaEvent_t* ev = nullptr, bool build_lists = false, bool after_prologue = false) {
   int L = 0;
@@ -300,8 +311,8 @@ static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, 
         k_eos<<<nblk(n), kBlock, 0, S.s>>>(a);
         L += 3;
       }
-      if (int rc = h16 ? launch_hydro_list<true>(a, n, S.s, S.list_shape)
-                       : launch_hydro_list<false>(a, n, S.s, S.list_shape))
+      if (int rc = h16 ? launch_hydro_list<true>(a, n, S.s, list_shape_now(S))
+                       : launch_hydro_list<false>(a, n, S.s, list_shape_now(S)))
         return rc;
       ++L;
     } else {
@@ -366,9 +377,9 @@ static int enqueue_reuse(SimImpl& S, StepArgs a, bool density, int* launches, cu
     }
     if (ev) WCSPH_CUDA(cudaEventRecord(ev[2], S.s));
     if (S.opt.precision == WCSPH_PREC_HALF2) {
-      if (int rc = launch_hydro_list<true>(a, n, S.s, S.list_shape)) return rc;
+      if (int rc = launch_hydro_list<true>(a, n, S.s, list_shape_now(S))) return rc;
     } else {
-      if (int rc = launch_hydro_list<false>(a, n, S.s, S.list_shape)) return rc;
+      if (int rc = launch_hydro_list<false>(a, n, S.s, list_shape_now(S))) return rc;
     }
     ++L;
     if (ev) WCSPH_CUDA(cudaEventRecord(ev[3], S.s));  // the dead tail stays in place
@@ -425,10 +436,11 @@ static int time_launches(SimImpl& S, int reps, F&& fn, float* ms) {
 
 // Autotuner: on the live instance set, time every block shape of the tiled
 // hydro kernel with probe passes (forces go to the diagnostic arrays, the
-// state is untouched) and keep the fastest.  The candidates share their
-// arithmetic exactly, so the choice never changes a result (an instance is
-// bit-identical alone and in a mix).  Re-tuned only when the particle count
-// crosses a power of two.
+// state is untouched) and keep the fastest; with lists, the scan's and the list
+// pass's shapes too.  The candidates share their arithmetic and its order
+// exactly, so what is timed never changes a result.  Re-tuned only when the
+// particle count crosses a power of two; between tunings the list pass keeps to
+// the order of the present count (list_shape_now).
 static int autotune(SimImpl& S) {
   if (!S.opt.autotune || S.opt.precision == WCSPH_PREC_FP32 || S.n_host <= 0) return 0;
   int bucket = 0;
@@ -464,9 +476,7 @@ static int autotune(SimImpl& S) {
     float best_list = 1e30f;
     const int fixed_list = S.opt.list_shape & 0xff, fixed_build = (S.opt.list_shape >> 8) & 0xff;
     int best_list_shape = fixed_list > 0 ? fixed_list - 1 : 0;
-    int sms = 0;
-    WCSPH_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S.opt.device));
-    for (int v : list_shape_candidates(n, h16, sms)) {
+    for (int v : list_shape_candidates(n, h16, S.sms)) {
       if (fixed_list > 0) break;
       int rc = time_launches(S, 3, [&]() {
         return h16 ? launch_hydro_list<true>(b, n, S.s, v) : launch_hydro_list<false>(b, n, S.s, v);
@@ -787,7 +797,9 @@ int wcsph_sim_create(const wcsph_sim_options* opt, wcsph_sim** out) {
     delete sim;
     return rc;
   };
-  if (cudaStreamCreateWithFlags(&S.s, cudaStreamNonBlocking) != cudaSuccess) return fail(WCSPH_E_CUDA);
+  if (cudaDeviceGetAttribute(&S.sms, cudaDevAttrMultiProcessorCount, opt->device) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&S.s, cudaStreamNonBlocking) != cudaSuccess)
+    return fail(WCSPH_E_CUDA);
   const size_t N = (size_t)opt->max_particles + 1;
   int rc = 0;
   for (SimArrays* A : {&S.buf_main, &S.buf_alt}) {
@@ -1539,8 +1551,8 @@ static int enqueue_probe_lists(SimImpl& S, int density_pass) {
       k_eos<<<nblk(n), kBlock, 0, S.s>>>(a);
     }
     const bool h16 = S.opt.precision == WCSPH_PREC_HALF2;
-    if (int rc = h16 ? launch_hydro_list<true>(a, n, S.s, S.list_shape)
-                     : launch_hydro_list<false>(a, n, S.s, S.list_shape))
+    if (int rc = h16 ? launch_hydro_list<true>(a, n, S.s, list_shape_now(S))
+                     : launch_hydro_list<false>(a, n, S.s, list_shape_now(S)))
       return rc;
   }
   WCSPH_CUDA(cudaGetLastError());
@@ -1667,7 +1679,7 @@ void* wcsph_sim_stream(wcsph_sim* sim) { return sim ? (void*)sim->impl.s : nullp
 int wcsph_sim_tuning(wcsph_sim* sim, int32_t* out4) {
   if (!sim || !out4) return WCSPH_E_INVALID;
   out4[0] = sim->impl.tile_shape;
-  out4[1] = sim->impl.list_shape;
+  out4[1] = list_shape_now(sim->impl);
   out4[2] = sim->impl.tuned_bucket;
   out4[3] = sim->impl.build_shape;
   return 0;

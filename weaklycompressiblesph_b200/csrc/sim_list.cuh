@@ -688,17 +688,23 @@ constexpr int kListShapes = 7;
 constexpr int kListShapeTPI[kListShapes] = {1, 2, 1, 2, 1, 1, 1};
 constexpr int kListShapeBlock[kListShapes] = {128, 128, 128, 128, 128, 128, 128};
 
-// The shapes timed for a solver of n particles: those of one summation order,
-// so that the choice among them never changes a result.  One or two threads per
-// particle is a rule on the waves of blocks (5 an SM): two where the waves of
-// the halved work take less time.  A wave of the two-thread shape takes 0.8
-// (FP32: its loop spills) or 0.6 (half2) of the other's: FP32 33,000 particles,
-// one wave either way, 21 against 22 us; 65,000, one wave against two, 30
-// against 34; half2 124,000, two against three, 58 against 58.
-inline std::vector<int> list_shape_candidates(int n, bool h16, int sms) {
+// Threads per particle of the list pass in a solver of n particles.  One and two
+// sum in different orders, so this is a rule on size and not a timing: two where
+// the waves of blocks (5 an SM) of the halved work take less time.  A wave of the
+// two-thread shape takes 0.8 (FP32: its loop spills) or 0.6 (half2) of the
+// other's: FP32 33,000 particles, one wave either way, 21 against 22 us; 65,000,
+// one wave against two, 30 against 34; half2 124,000, two against three, 58
+// against 58.
+inline int list_threads(int n, bool h16, int sms) {
   const long long blocks = (n + 127) / 128, slots = 5LL * sms;
   const long long w1 = (blocks + slots - 1) / slots, w2 = (2 * blocks + slots - 1) / slots;
-  if (h16 ? 3 * w2 < 5 * w1 : 4 * w2 < 5 * w1) return {1, 3};
+  return (h16 ? 3 * w2 < 5 * w1 : 4 * w2 < 5 * w1) ? 2 : 1;
+}
+
+// The shapes timed for a solver of n particles: those of one summation order,
+// so that the choice among them never changes a result.
+inline std::vector<int> list_shape_candidates(int n, bool h16, int sms) {
+  if (list_threads(n, h16, sms) == 2) return {1, 3};
   if (h16) return {0, 2, 4};
   return {0, 2};
 }
