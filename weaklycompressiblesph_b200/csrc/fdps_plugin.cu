@@ -235,14 +235,24 @@ __device__ __forceinline__ void walk_candidates(const uint32_t (*mask)[32], int 
   }
 }
 
+// A power of two near 1 / h^2: numerators carry it, so that the cross products of
+// walk_block stay in range whatever the unit of length.
+__device__ __forceinline__ float quotient_scale(float h) {
+  const int e = (int)(__float_as_uint(h) >> 23);
+  return __uint_as_float((unsigned)min(max(3 * 127 - 2 * e, 1), 254) << 23);
+}
+
 // Device-resident walks: hydro pair sum of kWalkChunk i-particles [ib, ib + nb)
 // of a walk over its j-records [j0, j1) (force.h:38-57; GPU variant
 // kernel.cu:241-280 when VSIG / GRAD select it).  The block's warps share the
 // words of a tile; a lane evaluates its own i's candidates, the warps' sums
-// are added in order.  VSIG: v_sig is max(-mu) over every j of the walk, in
-// support or not (kernel.cu:263): each lane keeps the numerator and denominator
-// of the most negative quotient per half, compared by fast quotients (within
-// 2 ulp), and divides them exactly once at the end.
+// are added in order.  VSIG: v_sig is max(-mu) over every j of the walk with
+// r^2 > 0, in support or not (kernel.cu:263): each lane keeps the numerator and
+// denominator of the most negative quotient per half and divides them once at
+// the end.  Quotients are compared by their cross products, exactly: n d' < n' d
+// as the two products' remainders from the rounded n' d, which fma gives without
+// error.  (Rounding is monotone, so the largest quotient rounds to the largest
+// rounded one.)
 template <int VSIG, int GRAD, class Rec>
 __device__ __forceinline__ void walk_block(const Rec& R, int ib, int nb, int j0, int j1, const WalkPair& pp) {
   __shared__ WalkSmem<VSIG ? 8 : 4, 5> S;
@@ -250,11 +260,13 @@ __device__ __forceinline__ void walk_block(const Rec& R, int ib, int nb, int j0,
   const int i = ib + min(lane, nb - 1);
   const float4 a = R.ia(i), b = R.ib(i), c = R.icr(i);
   const GradH gi = grad_h(a.w);
-  const f2 IX = dup(a.x), IY = dup(a.y), IZ = dup(a.z), IH = dup(a.w);
+  const f2 IX = dup(a.x), IY = dup(a.y), IZ = dup(a.z);
   const f2 VX = dup(b.x), VY = dup(b.y), VZ = dup(b.z), EH = dup(pp.eps * a.w);
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  f2 NUM = 0ull, DEN = dup(1.0f);
-  float qa = 0.0f, qb = 0.0f, vs = 0.0f;
+  const float scale = quotient_scale(a.w);
+  const f2 SC = dup(scale), IHS = dup(scale * a.w);
+  f2 NUM = 0ull, DEN = dup(1.0f);  // the numerator negated
+  float vs = 0.0f;
   for (int jb = j0; jb < j1; jb += kWalkTile) {
     const int nt = min(kWalkTile, j1 - jb), nt32 = (nt + 31) & ~31;
     __syncthreads();  // the previous tile's readers are done
@@ -290,11 +302,11 @@ __device__ __forceinline__ void walk_block(const Rec& R, int ib, int nb, int j0,
           const f2 HJ = tile2(S.t[3], u);
           const f2 DV = fma2(DZ, sub2(VZ, tile2(S.t[6], u)), fma2(DY, sub2(VY, tile2(S.t[5], u)),
                                                                    mul2(DX, sub2(VX, tile2(S.t[4], u)))));
-          const f2 N = mul2(add2(IH, HJ), DV), D = fma2(EH, HJ, R2);  // 2 mu = N / D where N < 0
-          const f2 Q = mul2(pk(fminf(lo(N), 0.0f), fminf(hi(N), 0.0f)), rcp2(D));
-          const bool t0 = lo(Q) < qa, t1 = hi(Q) < qb;
-          qa = t0 ? lo(Q) : qa, qb = t1 ? hi(Q) : qb;
-          NUM = pk(t0 ? lo(N) : lo(NUM), t1 ? hi(N) : hi(NUM));
+          const f2 N = mul2(fma2(HJ, SC, IHS), DV), D = fma2(EH, HJ, R2);  // 2 mu scale = N / D where N < 0
+          const f2 P = mul2(NUM, D), X = fma2(N, DEN, P);
+          const bool t0 = lo(R2) > 0.0f && lo(X) < __fmaf_rn(-lo(NUM), lo(D), lo(P));
+          const bool t1 = hi(R2) > 0.0f && hi(X) < __fmaf_rn(-hi(NUM), hi(D), hi(P));
+          NUM = pk(t0 ? -lo(N) : lo(NUM), t1 ? -hi(N) : hi(NUM));
           DEN = pk(t0 ? lo(D) : lo(DEN), t1 ? hi(D) : hi(DEN));
         }
       }
@@ -307,7 +319,10 @@ __device__ __forceinline__ void walk_block(const Rec& R, int ib, int nb, int j0,
       walk_pair<GRAD>(a, b, c, gi, J, V, R.jcr(jb + u), pp, acc);
     });
   }
-  if (VSIG) vs = fmaxf(0.0f, fmaxf(-(0.5f * lo(NUM) / lo(DEN)), -(0.5f * hi(NUM) / hi(DEN))));
+  if (VSIG) {
+    const float half = 0.5f / scale;
+    vs = fmaxf(0.0f, fmaxf(half * lo(NUM) / lo(DEN), half * hi(NUM) / hi(DEN)));
+  }
 #pragma unroll
   for (int k = 0; k < 4; ++k) S.res[warp][k][lane] = acc[k];
   S.res[warp][4][lane] = vs;
