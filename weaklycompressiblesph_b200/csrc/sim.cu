@@ -72,6 +72,7 @@ struct SimImpl {
   bool appended = false;       // particles were appended after the last pass (its live count is stale)
   int key_bits = 1;
   long long total_cells = 0;
+  float cell_load = 0.f;       // particles in a full cell, over the active instances
   bool any_density = false;
   int tile_shape = 0;          // tiled pair-kernel shape, chosen by the autotuner
   int list_shape = 0;          // list-pass launch shape (kListShapes), chosen by the autotuner (list_shape_now)
@@ -152,6 +153,7 @@ static int upload_tables(SimImpl& S) {
 static int rebuild_tables(SimImpl& S) {
   uint64_t key = 0;
   long long cells = 0;
+  double particles = 0.0, full_cells = 0.0;
   S.any_density = false;
   for (size_t k = 0; k < S.inst.size(); ++k) {
     HostInst& I = S.inst[k];
@@ -164,6 +166,8 @@ static int rebuild_tables(SimImpl& S) {
     P.cell_base = (int)cells;
     key += (uint64_t)1 << (3 * I.bits);
     cells += (long long)I.ncell[0] * I.ncell[1] * I.ncell[2];
+    particles += I.n;
+    full_cells += I.n * (I.desc.mass / I.desc.rho0) / ((double)I.cell[0] * I.cell[1] * I.cell[2]);
     if (I.desc.density_mode != WCSPH_DENSITY_CONTINUITY) S.any_density = true;
   }
   if (key >= 0xffffffffull) {
@@ -175,6 +179,7 @@ static int rebuild_tables(SimImpl& S) {
     return WCSPH_E_CAPACITY;
   }
   S.total_cells = cells;
+  S.cell_load = full_cells > 0.0 ? (float)(particles / full_cells) : 0.f;
   int bits = 1;
   while (bits < 32 && ((uint64_t)1 << bits) <= key) ++bits;  // DeadKey & mask must exceed every live key
   S.key_bits = bits;
@@ -292,13 +297,13 @@ static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, 
     // scan reads positions only, and the EoS records it gathers do not enter
     // the lists.  Other passes search the cells for the density.
     if (density && !build_lists) {
-      if (int rc = launch_cell_plain<PLAIN_DENSITY>(a, n, S.s)) return rc;
+      if (int rc = launch_plain<PLAIN_DENSITY>(a, n, S.cell_load, S.s)) return rc;
       k_eos<<<nblk(n), kBlock, 0, S.s>>>(a);
       L += 2;
     }
     if (ev) WCSPH_CUDA(cudaEventRecord(ev[2], S.s));
     if (S.opt.precision == WCSPH_PREC_FP32) {
-      if (int rc = launch_cell_plain<PLAIN_HYDRO>(a, n, S.s)) return rc;
+      if (int rc = launch_plain<PLAIN_HYDRO>(a, n, S.cell_load, S.s)) return rc;
     } else if (build_lists) {  // the scan writes the lists, the list pass sums them
       const bool h16 = S.opt.precision == WCSPH_PREC_HALF2;
       if (int rc = h16 ? launch_list_scan<true>(a, n, S.s, S.build_shape)
@@ -323,7 +328,7 @@ static int enqueue_pass(SimImpl& S, StepArgs a, bool density, bool init_filter, 
     if (init_filter) {
       StepArgs b = a;
       b.init_filter = 1;
-      if (int rc = launch_cell_plain<PLAIN_DENSITY>(b, n, S.s)) return rc;
+      if (int rc = launch_plain<PLAIN_DENSITY>(b, n, S.cell_load, S.s)) return rc;
       k_apply_init_filter<<<nblk(n), kBlock, 0, S.s>>>(b);
       L += 2;
     }

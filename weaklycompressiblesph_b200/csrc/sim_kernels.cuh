@@ -396,11 +396,11 @@ __device__ __forceinline__ bool wants_force(const InstParams& P, const InstDyn& 
   return ph == PH_INIT || ph == PH_PROBE || (ph == PH_STEP && d.dt_cur > 0.0f);
 }
 
-// The cell search of one particle: calls body(q, r2, code) for every in-support
-// j (0 < r2 < (2h)^2, FP32 predicate of the oracle), neighbour cells in the order
-// z, y, x and slots in order within a cell; code is the periodic image code of
-// the tiled kernel's queue entries ((sx+1) + 3 (sy+1) + 9 (sz+1) in units of the
-// box).
+// The cell search of one particle: calls body(q, J, dx, dy, dz, r2, code) for every
+// in-support j (0 < r2 < (2h)^2, FP32 predicate of the oracle; J its jr.a),
+// neighbour cells in the order z, y, x and slots in order within a cell; code is
+// the periodic image code of the tiled kernel's queue entries ((sx+1) + 3 (sy+1) +
+// 9 (sz+1) in units of the box).
 template <typename Body>
 __device__ __forceinline__ void for_each_neighbor(const StepArgs& a, const InstParams& P, float xi, float yi, float zi,
                                                   Body&& body) {
@@ -431,7 +431,7 @@ __device__ __forceinline__ void for_each_neighbor(const StepArgs& a, const InstP
           const float dy = __fsub_rn(yi, __fadd_rn(J.y, sy));
           const float dz = __fsub_rn(zi, __fadd_rn(J.z, sz));
           const float r2 = dist2(dx, dy, dz);
-          if (r2 > 0.0f && r2 < H2) body(q, r2, code);
+          if (r2 > 0.0f && r2 < H2) body(q, J, dx, dy, dz, r2, code);
         }
       }
     }
@@ -439,9 +439,23 @@ __device__ __forceinline__ void for_each_neighbor(const StepArgs& a, const InstP
 }
 
 // ---------------------------------------------------------- density pass
+// Density of particle p by its own cell search (k_density_plain's sums).
+__device__ __forceinline__ void search_density(const StepArgs& a, const InstParams& P, int p, int kind) {
+  const float4 I = a.jr[p].a;
+  const float rho_i = a.jr[p].b.w;
+  float sum = 0.5f, one = 0.5f / rho_i;  // self term: w(0) = 1/2
+  const float iH = P.inv_H;
+  const bool shep = kind == 2;
+  for_each_neighbor(a, P, I.x, I.y, I.z, [&](int q, const float4&, float, float, float, float r2, uint32_t) {
+    const float w = spline_w(sqrtf(r2) * iH);
+    sum += w;
+    if (shep) one += w / __ldg(&a.jr[q].b.w);
+  });
+  a.rho_new[p] = shep ? sum / one : P.mass * P.Kw * sum;
+}
+
 // Density pass of a list build for the particles whose list overflowed, over
-// the cells (k_density_plain's sums; every other particle reads its list,
-// k_density_list).
+// the cells (every other particle reads its list, k_density_list).
 __global__ void k_density_overflow(StepArgs a) {
   if (a.dens_any && !*a.dens_any) return;  // no density pass in this launch
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -454,17 +468,7 @@ __global__ void k_density_overflow(StepArgs a) {
   // an instance that keeps its lists in a partial build: its cells are those
   // of its build positions, so its density pass reads the lists (k_density_list)
   if (a.inst_keep && a.list_flags[kLfPartial] != 0u && a.inst_keep[inst]) return;
-  const float4 I = a.jr[p].a;
-  const float rho_i = a.jr[p].b.w;
-  float sum = 0.5f, one = 0.5f / rho_i;  // self term: w(0) = 1/2
-  const float iH = P.inv_H;
-  const bool shep = kind == 2;
-  for_each_neighbor(a, P, I.x, I.y, I.z, [&](int q, float r2, uint32_t) {
-    const float w = spline_w(sqrtf(r2) * iH);
-    sum += w;
-    if (shep) one += w / __ldg(&a.jr[q].b.w);
-  });
-  a.rho_new[p] = shep ? sum / one : P.mass * P.Kw * sum;
+  search_density(a, P, p, kind);
 }
 
 // Refresh the j-records of particles whose density was just recomputed.

@@ -565,7 +565,7 @@ __device__ __forceinline__ void hydro_list_body(const StepArgs& a) {
         // next step, so no list step ever sees it): sum over the cell search
         // of the build's cell table instead, one j at a time.
         for_each_neighbor(a, P, R.a.x, R.a.y, R.a.z,
-                          [&](int q, float, uint32_t code) {
+                          [&](int q, const float4&, float, float, float, float, uint32_t code) {
                             const JRec Rq = ld_jrec(&a.jr[q]);
                             const float cq = g7 ? lo(snds7_2(dup(Rq.b.w), RHO0, IRHO0, C0)) : __ldg(&a.jC[q]);
                             pair2<false>(P, C, I, Rq, R, code, 13u, dup(cq), true, false, AX, AY, AZ, DS, vsa, vsb,

@@ -322,8 +322,98 @@ __global__ void __launch_bounds__(32, 12) k_density_plain(const __grid_constant_
   cell_pass<PLAIN_DENSITY>(a, S);
 }
 
+// The same passes with one thread per particle that walks the 27 cells itself:
+// candidates are read from the caches, a warp's lanes diverge, but nothing is
+// paid per cell.  Every term and addition is that of the cell passes, to the bit.
+__global__ void __launch_bounds__(256) k_density_particle(const __grid_constant__ StepArgs a) {
+  if (a.dens_any && !*a.dens_any) return;  // no density pass in this launch
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= *a.n_alive) return;
+  const int inst = a.alt.flags[p] & kInstMask;
+  const InstParams& P = a.params[inst];
+  const int kind = density_kind(a, P, a.dyn[inst], a.phase[inst]);
+  if (kind) search_density(a, P, p, kind);
+}
+
+__global__ void __launch_bounds__(256) k_hydro_particle(const __grid_constant__ StepArgs a) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  int inst = 0;
+  float dt_cand = 0.0f;
+  bool dt_valid = false;
+  unsigned cnt = 0;
+  if (p < *a.n_alive) {
+    const uint32_t f = a.alt.flags[p];
+    inst = f & kInstMask;
+    const InstParams& P = a.params[inst];
+    const int ph = a.phase[inst];
+    if (wants_force(P, a.dyn[inst], ph)) {
+      const float4 I = a.jr[p].a, IB = a.jr[p].b;
+      const float ci = a.jC[p];
+      float ax = 0.f, ay = 0.f, az = 0.f, ndsum = -0.f, vsig = 0.f;
+      const float nih = -P.inv_H, nkg = -P.Kg, eh2 = P.eh2, h = P.h, beta = P.beta, nah = -(P.alpha * 0.5f), nnu4 = -P.nu4;
+      const int vs = P.vsig_mode;
+      for_each_neighbor(a, P, I.x, I.y, I.z, [&](int q, const float4& J, float dx, float dy, float dz, float r2, uint32_t) {
+        ++cnt;
+        const float4 B = __ldg(&a.jr[q].b);
+        const float cj = __ldg(&a.jC[q]);
+        // pair_terms, operation by operation
+        const float rinv = rsqrtf(r2), s = __fmul_rn(r2, rinv);
+        const float A1 = fmaxf(__fmaf_rn(s, nih, 1.0f), 0.0f), B1 = fmaxf(__fmaf_rn(s, nih, 0.5f), 0.0f);
+        const float F = __fmaf_rn(__fmul_rn(12.0f, B1), B1, __fmul_rn(__fmul_rn(-3.0f, A1), A1));
+        const float ng = __fmul_rn(__fmul_rn(F, nkg), rinv);
+        const float dvx = __fsub_rn(IB.x, B.x), dvy = __fsub_rn(IB.y, B.y), dvz = __fsub_rn(IB.z, B.z);
+        const float drdv = __fmaf_rn(dz, dvz, __fmaf_rn(dx, dvx, __fmul_rn(dy, dvy)));
+        const float rden = __frcp_rn(__fadd_rn(r2, eh2)), rs = __frcp_rn(__fadd_rn(IB.w, B.w));
+        const float mu = drdv < 0.0f ? __fmul_rn(__fmul_rn(h, drdv), rden) : 0.0f;
+        const float av = __fmul_rn(__fmul_rn(__fmaf_rn(beta, mu, __fmul_rn(nah, __fadd_rn(ci, cj))), mu), 2.0f);
+        const float npg = __fmul_rn(__fmaf_rn(av, rs, __fadd_rn(I.w, J.w)), ng);
+        const float visc = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(nnu4, ng), r2), rs), rden);
+        ax = __fadd_rn(ax, __fmaf_rn(visc, dvx, __fmul_rn(npg, dx)));
+        ay = __fadd_rn(ay, __fmaf_rn(visc, dvy, __fmul_rn(npg, dy)));
+        az = __fadd_rn(az, __fmaf_rn(visc, dvz, __fmul_rn(npg, dz)));
+        ndsum = __fmaf_rn(ng, drdv, ndsum);
+        vsig = fmaxf(vsig, vs ? -mu : mu);
+      });
+      finish_hydro(a, p, P, inst, ph, f, ax, ay, az, -ndsum, vsig, cnt, dt_cand, dt_valid);
+      if (f & kGhostBit) cnt = 0;  // pairs are counted for owned particles only
+    } else {
+      copy_state(a, p);
+    }
+  } else if (p < a.n_host) {
+    copy_state(a, p);  // the dead tail
+  }
+  dt_min(a.dyn, inst, dt_cand, dt_valid);
+  unsigned long long pairs = cnt;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+  if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(a.pair_count, pairs);
+}
+
+// Which of the two for n particles with `load` of them in a full cell (the cell's
+// volume over a particle's, m / rho0).  A cell costs a warp 2 ns + 0.9 ns a particle
+// of GPU time (hydro, large solvers), a thread's walk 0.3 ns + 0.07 ns x load, but at
+// least 35 us + 8 us x load from end to end.  Hydro pass, us, cell / particle, by load
+// 1.4, 4.5, 6, 9, 11, 14.5, 19 on jittered lattices:
+//   64,000     159/46   92/80   92/86    79/113   84/128   82/161   88/197
+//   125,000    300/52  180/111 153/111  136/136  144/172  151/221  160/258
+//   512,000   1207/158 685/312 622/328  528/368  557/499  599/674  548/773
+//   1,728,000 4329/465 2368/972 2083/1019 1829/1086 1883/1552 1966/2122 1946/2408
+// Density pass:
+//   64,000     105/45   69/77   70/81    62/96    73/108   73/129   75/154
+//   512,000    738/112 453/207 428/210  384/218  406/290  425/372  385/433
+//   1,728,000 2534/297 1527/590 1404/593 1273/590 1324/828 1376/1075 1348/1212
+inline bool thread_per_particle(int pass, int n, float load) {
+  return pass == PLAIN_HYDRO ? load <= 12.0f && n >= 12000.0f * load : load <= 16.0f + n / 4.0e5f && n >= 19000.0f * load;
+}
+
 template <int PASS>
-inline int launch_cell_plain(const StepArgs& a, int n, cudaStream_t s) {
+inline int launch_plain(const StepArgs& a, int n, float load, cudaStream_t s) {
+  if (thread_per_particle(PASS, n, load)) {
+    auto kern = PASS == PLAIN_HYDRO ? k_hydro_particle : k_density_particle;
+    kern<<<(n + 255) / 256, 256, 0, s>>>(a);
+    WCSPH_CUDA(cudaGetLastError());
+    return 0;
+  }
   static TiledLaunch L[16];
   int dev = 0;
   WCSPH_CUDA(cudaGetDevice(&dev));
