@@ -88,15 +88,18 @@ struct ReadField {
   int width;
 };
 
-// Ring of host blocks the pieces of a read pass through, allocated by the
-// first read for the largest one the solver can have, at most kBlockBytes each
-// (1.6 M particles, 72 MB: 4.6 ms with blocks of 8 MB, 7.3 with 4), and given
-// back with the solver.  Blocks above kSecondBytes are huge pages registered with
-// the device at once: 12 MB cost 0.8 ms that way and 5.6 ms from cudaMallocHost.
-// Smaller ones are registered by the second read (0.4 ms: more than one read
-// gains by it; 12,600 particles: 0.22 ms a read, 0.10 registered), and those
-// below kPinBytes never.  Unregistered, and where registering fails, ordinary
-// memory serves; copies into it are synchronous.
+// Ring of host blocks the pieces of a read pass through, given back with the
+// solver.  Its full size is for the largest read the solver can have, at most
+// kBlockBytes a block (1.6 M particles, 72 MB: 4.6 ms with blocks of 8 MB, 7.3
+// with 4), registered with the device.  That costs 0.4 to 2 ms once, at times more
+// (12 MB of huge pages 0.8 ms; cudaMallocHost 5.6), and is done by the read with
+// which the reads so far have brought a quarter of the ring's bytes: by the first
+// one of a large instance, by the second where blocks are up to kSecondBytes
+// (12,600 particles: 0.22 ms a read, 0.10 registered), late where a large solver is
+// asked for a few particles (300 of 4 M: a first read of 2 ms and more with the
+// full ring, 0.15 without).  Until then, where blocks are below kPinBytes, and where
+// registering fails, ordinary memory of the read's own size serves; copies into it
+// are synchronous.
 class ReadRing {
  public:
   ~ReadRing() { release(); }
@@ -110,11 +113,7 @@ class ReadRing {
       int field, i0, i1;  // field -1: cover
       size_t off;
     };
-    // 45 bytes a particle and the alignment of a handful of pieces: a quarter of
-    // that a block, but 1 MB in one
-    const long long whole = 48 * n_max + 4096;
-    const long long block = std::min<long long>(kBlockBytes, std::max<long long>(whole / 4, std::min<long long>(whole, 1 << 20)));
-    if (int rc = reserve((size_t)(block + 4095) / 4096 * 4096)) return rc;
+    if (int rc = reserve(s, n, n_max)) return rc;
     // Pieces in order, cut into batches of one block each.
     std::vector<std::vector<Piece>> batch(1);
     size_t used = kHead;  // the first block starts with the count of missing particles
@@ -196,15 +195,11 @@ class ReadRing {
   }
 
   void release() {
-    if (pinned_) cudaHostUnregister(mem_);
-    free(mem_);
+    drop();
     for (cudaEvent_t& e : ev_) {
       if (e) cudaEventDestroy(e);
       e = nullptr;
     }
-    mem_ = nullptr;
-    pinned_ = false;
-    bytes_ = 0;
   }
 
  private:
@@ -223,29 +218,50 @@ class ReadRing {
       body(i0 + (int)((long long)(i1 - i0) * k / t), i0 + (int)((long long)(i1 - i0) * (k + 1) / t));
   }
 
-  int reserve(size_t bytes) {
+  static size_t read_bytes(long long n) { return 48 * (size_t)n + 4096; }  // 45 a particle and a few pieces' alignment
+  // A block of the ring for reads of n particles: a quarter of one, but 1 MB in one block.
+  static size_t block_bytes(long long n) {
+    const size_t whole = read_bytes(n);
+    const size_t b = std::min<size_t>(kBlockBytes, std::max<size_t>(whole / 4, std::min<size_t>(whole, 1 << 20)));
+    return (b + 4095) / 4096 * 4096;
+  }
+
+  int reserve(cudaStream_t s, int n, long long n_max) {
     for (cudaEvent_t& e : ev_)
       if (!e) WCSPH_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    if (bytes_) {
-      if (!pinned_ && reads_++ == 0) pin();
-      return 0;
+    if (full_) return 0;
+    const size_t full = block_bytes(n_max);
+    ++reads_;
+    total_ += read_bytes(n);
+    const bool now = full >= kPinBytes && 4 * total_ >= kBlocks * full && (full > kSecondBytes || reads_ > 1);
+    const size_t want = now || full <= kSecondBytes ? full : block_bytes(n);
+    if (bytes_ < want) {
+      if (mem_) WCSPH_CUDA(cudaStreamSynchronize(s));  // a read that failed may have left copies in flight
+      drop();
+      const size_t all = (want * kBlocks + kHuge - 1) / kHuge * kHuge;
+      mem_ = static_cast<char*>(now || want >= kPinBytes ? aligned_alloc(kHuge, all) : malloc(want * kBlocks));
+      if (!mem_) {
+        set_error("read: %zu bytes of host memory are not to be had", want * kBlocks);
+        return WCSPH_E_NOMEM;
+      }
+      bytes_ = want;
     }
-    const size_t all = bytes < kPinBytes ? bytes * kBlocks : (bytes * kBlocks + kHuge - 1) / kHuge * kHuge;
-    mem_ = static_cast<char*>(bytes < kPinBytes ? malloc(all) : aligned_alloc(kHuge, all));
-    if (!mem_) {
-      set_error("read: %zu bytes of host memory are not to be had", all);
-      return WCSPH_E_NOMEM;
-    }
-    bytes_ = bytes;
-    if (bytes > kSecondBytes) {
-      ++reads_;
+    if (now) {
+      full_ = true;
       pin();
     }
     return 0;
   }
 
+  void drop() {
+    if (pinned_) cudaHostUnregister(mem_);
+    free(mem_);
+    mem_ = nullptr;
+    pinned_ = full_ = false;
+    bytes_ = 0;
+  }
+
   void pin() {
-    if (bytes_ < kPinBytes) return;
     const size_t all = (bytes_ * kBlocks + kHuge - 1) / kHuge * kHuge;
     if (bytes_ > kSecondBytes) {
       madvise(mem_, all, MADV_HUGEPAGE);
@@ -257,8 +273,10 @@ class ReadRing {
 
   char* mem_ = nullptr;
   cudaEvent_t ev_[kBlocks] = {};
-  size_t bytes_ = 0;  // per block; the same in every read of a solver
-  int reads_ = 0;     // since the blocks were allocated, until they are registered
+  size_t bytes_ = 0;      // per block
+  size_t total_ = 0;      // bytes of the reads so far
+  long long reads_ = 0;
+  bool full_ = false;     // full size, and registered if it can be
   bool pinned_ = false;
 };
 
