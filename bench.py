@@ -767,10 +767,11 @@ def hbm_roofline(workload, prec, n, dev, peak, peak_kind):
 
 def l1_roofline(workload, prec, dev):
     """The FP32 list pass is bound by the L1 data pipe that delivers its
-    gathers (the half2 pass about as much by issue).  Per list entry it needs
-    one list word and one j-record (half2: the compact record and P/rho^2): at
-    128 B per L1 wavefront that is (4 + record bytes) / 128 wavefronts at least.  The
-    measured L1 load wavefronts of one launch come from the ncu capture
+    gathers (the half2 pass by issue).  Its global loads need at least one
+    j-record per list entry (half2: the compact record and P/rho^2) and, where
+    rows come by plain loads (half2; the FP32 pass copies them past the L1), the
+    list word: at 128 B per L1 wavefront (word + record bytes) / 128 wavefronts.
+    The measured L1 load wavefronts of one launch come from the ncu capture
     summarised in profiles/hydro_list_l1.json; entries and true pairs are this
     run's."""
     t = _profile_json("hydro_list_l1.json")
@@ -781,7 +782,7 @@ def l1_roofline(workload, prec, dev):
     if not r:
         return None
     entries, pairs = lists["entries"], dev["pairs_per_step"]
-    need = entries * (4 + r["record_bytes"]) / 128.0
+    need = entries * (r["list_word_bytes"] + r["record_bytes"]) / 128.0
     return {"bound": "l1", "wavefronts_per_launch": r["wavefronts"], "min_wavefronts_per_launch": need,
             "frac": need / r["wavefronts"], "wavefronts_per_pair": r["wavefronts"] / pairs,
             "entries_per_pair": entries / pairs, "record_bytes": r["record_bytes"],
