@@ -294,7 +294,7 @@ __device__ __forceinline__ void walk_block(const Rec& R, int ib, int nb, int j0,
     int words = 0;
     for (int u0 = 32 * warp; u0 < nt32; u0 += 32 * kWalkWarps, ++words) {
       uint32_t m = 0;
-#pragma unroll 8
+#pragma unroll  // the whole word: 749 us a call for 0.3 M particles, 766 by eight pairs
       for (int u = u0; u < u0 + 32; u += 2) {
         f2 DX, DY, DZ;
         const f2 R2 = scan2(S.t, u, IX, IY, IZ, NB2, DX, DY, DZ, m);
