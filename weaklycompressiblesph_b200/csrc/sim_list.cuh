@@ -1,9 +1,9 @@
 // Neighbour-list steps (wcsph_sim_options.list_interval > 0).
 //
-// A build step is an ordinary step whose tiled kernel only scans: it writes,
-// for every particle, the candidates within 2h + skin (the list radius), and
-// the pair terms are summed by the list pass (k_hydro_list); its permutation
-// records the positions x0 the lists refer to.  The steps up to the next
+// A build step is an ordinary step with a scan (k_list_scan, sim_scan.cuh) in the
+// place of the hydro pass: it writes, for every particle, the candidates within
+// 2h + skin (the list radius), and the pair terms are summed by the list pass
+// (k_hydro_list); its permutation records the positions x0 the lists refer to.  The steps up to the next
 // build skip the binning sort and the candidate scan:
 //   k_kick_refresh  KDK first half in place (periodic wrapping waits for the
 //                 next build, so that the lists' image shifts stay valid),
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(128) k_density_list(StepArgs a) {
   const float4 I = a.jr[p].a;
   const float rho_i = a.jr[p].b.w;
   // a list that overflowed at this step's build: k_density_overflow sums it over
-  // the cell search (k_density_overflow), and the next step builds again
+  // the cell search, and the next step builds again
   if (a.list_cnt[p] > a.list_max) return;
   const int n = min(a.list_cnt[p], a.list_max);
   const uint4* row = list_row(a, p);
@@ -508,16 +508,17 @@ __device__ __forceinline__ void h16_pair2(const StepArgs& a, const InstParams& P
 // particle walk its list row, each taking every TPI-th group of four entries
 // (one 16-byte load), and sum two entries at a time in the f32x2 halves of
 // pair2, support tested per entry; the TPI partial sums are combined with
-// shuffles, and no shared memory is used.  For gamma = 7 the sound speed of j
-// is recomputed from its density (snds7_2, the stored value bit for bit)
-// instead of gathered: one gather per entry fewer.  MINB is the launch
-// bound's blocks per SM (it sets the register budget).  With TPI = 1 every
-// sum runs in list order; TPI = 2 changes the summation order (the results
-// agree to FP32 rounding).  The half2 pass (H16) reads every group of four
+// shuffles.  The FP32 pass's rows come through shared memory (RowStream).  For
+// gamma = 7 the sound speed of j is recomputed from its density (snds7_2, the
+// stored value bit for bit) instead of gathered: one gather per entry fewer.
+// MINB is the launch bound's blocks per SM (it sets the register budget).  With
+// TPI = 1 every sum runs in list order; TPI = 2 changes the summation order (the
+// results agree to FP32 rounding).  The half2 pass (H16) reads every group of four
 // whole: rows are padded with the padding slot's entry (k_list_pad_slot);
 // OFT and POR choose how it gets the neighbour-cell offsets and P/rho^2
 // (h16_pair2).  The FP32 pass keeps its per-entry selects of i's own record
-// for the entries past n, which fit its 96 registers without spilling.
+// for the entries past n (without them the loop before the row stream spilled
+// 32 bytes and took 0.652 against 0.547 ms).
 template <bool H16, int TPI, bool OFT = false, bool POR = false>
 __device__ __forceinline__ void hydro_list_body(const StepArgs& a) {
   const unsigned full = 0xffffffffu;
@@ -613,8 +614,7 @@ __device__ __forceinline__ void hydro_list_body(const StepArgs& a) {
           sum(e);
         }
       } else {
-        // idle halves past n read i's own record (weight 0): this loop keeps
-        // its selects, which leave the FP32 pass within 96 registers
+        // idle halves past n read i's own record (weight 0)
         const uint32_t self = (uint32_t)p | (13u << 27);
         __shared__ uint4 s_rows[kRowStages][128];
         RowStream<TPI> row(list_row(a, p), s_rows, n, sub);
@@ -677,13 +677,15 @@ __global__ void __launch_bounds__(128, MINB) k_hydro_list(StepArgs a) {
 
 // Launch shapes of the list pass the autotuner chooses among: (threads per
 // particle, blocks of 128 per SM of the launch bound, which sets the register
-// budget: 96 or 128).  Shapes 0 and 2 sum in one order (bit-identical
+// budget: 96 or 128; at 96 the loops spill, FP32 32 bytes in shape 0 and 56 in 3,
+// half2 4 and 64, at 128 none does).  Shapes 0 and 2 sum in one order (bit-identical
 // results), shapes 1 and 3 in another.  Shapes 4-6 are shape 0 with the half2
 // pass's other ways to the offsets and P/rho^2 (h16_pair2 OFT, POR): 4 the
 // shared offset table, bit-identical to 0; 5 and 6 recompute P/rho^2 (FP32
 // rounding of 0), with shifts or with the table.  In the FP32 pass they are
-// shape 0.  (On the 1.6M dam break the half2 pass takes 0.566 ms in shape 0,
-// 0.615 with the table, 0.578 and 0.589 recomputing P/rho^2.)
+// shape 0.  (On the 1.6M dam break the half2 pass took 0.566 ms in shape 0,
+// 0.615 with the table, 0.578 and 0.589 recomputing P/rho^2; since its loop was
+// peeled 0.552 in shape 0, the FP32 pass 0.509.)
 constexpr int kListShapes = 7;
 constexpr int kListShapeTPI[kListShapes] = {1, 2, 1, 2, 1, 1, 1};
 constexpr int kListShapeBlock[kListShapes] = {128, 128, 128, 128, 128, 128, 128};
@@ -691,8 +693,7 @@ constexpr int kListShapeBlock[kListShapes] = {128, 128, 128, 128, 128, 128, 128}
 // Threads per particle of the list pass in a solver of n particles.  One and two
 // sum in different orders, so this is a rule on size and not a timing: two where
 // the waves of blocks (5 an SM) of the halved work take less time.  A wave of the
-// two-thread shape takes 0.8 (FP32: its loop spills) or 0.6 (half2) of the
-// other's: FP32 33,000 particles, one wave either way, 21 against 22 us; 65,000,
+// two-thread shape takes 0.8 (FP32) or 0.6 (half2) of the other's: FP32 33,000 particles, one wave either way, 21 against 22 us; 65,000,
 // one wave against two, 30 against 34; half2 124,000, two against three, 58
 // against 58.
 inline int list_threads(int n, bool h16, int sms) {

@@ -10,7 +10,8 @@
 // their order are those of a loop over every candidate, so that the block shape
 // and the staging never change a bit.
 //
-// Against one thread per particle that walked the 27 cells itself, a step's
+// Against one thread per particle that walks the 27 cells itself (k_hydro_particle,
+// kept for large solvers with few particles a cell: thread_per_particle), a step's
 // hydro pass: dam break of 12,600 particles 163 -> 39 us, of 54,500 186 -> 76,
 // of 477,000 559 -> 468, of 1.25 M 1395 -> 1250; cells of 83 particles (8,100 in
 // all) 492 -> 340.  Density pass of a lattice of 64,000: 149 -> 81 us.
@@ -49,9 +50,9 @@ struct PlainI {
   f2 NIH, NKG, EH2, H, BETA, NAH, NNU4;  // -1/2h, -Kg, eps h^2, h, beta, -alpha/2, -4 nu
 };
 // The terms of two pairs, one per half (force.h:38-57 for uniform h, m, nu): NG
-// is minus the gradient factor.  Every product, sum and fma is the one that the
-// scalar expression (visc * dvx - pg * dx and so on) is compiled to, so that the
-// terms are those of a scalar loop to the bit.
+// is minus the gradient factor.  Which products are fused into an fma is written
+// out here, and again one pair at a time in k_hydro_particle: the two agree to the
+// bit.
 struct PairTerms {
   f2 R2, X, Y, Z, NG, DRDV, MU;
 };

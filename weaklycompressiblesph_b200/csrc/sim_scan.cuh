@@ -25,7 +25,7 @@
 // The rows hold the candidates in the order of the cell search, whatever the
 // block shape.
 //
-// Measured on a dam break under way (1.6M particles, 147M entries): 0.764 ms
+// Measured on a dam break under way (1.6M particles, 147M entries): 0.72-0.76 ms
 // a build, 1.244 ms with a lane per particle walking all 27 cells' candidates
 // and storing single words (32 separate sectors a store); periodic lattice of
 // 1M: 0.625 against 0.942 ms; half2 lists of 0.5M: 0.322 against 0.429 ms.

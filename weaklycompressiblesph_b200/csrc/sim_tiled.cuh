@@ -76,12 +76,6 @@ __device__ __forceinline__ float warp_max_f(float v) {
   return r;
 }
 
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
 // Butterfly reduce-scatter of 8 per-lane sums: returns, in every lane, the
 // warp total of slot ((lane >> 2) & 7).  9 shuffles instead of 40.
 __device__ __forceinline__ float butterfly8(const float v[8], int lane) {
