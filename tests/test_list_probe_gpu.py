@@ -59,6 +59,30 @@ def test_probe_of_a_finished_instance(prec, native, oracle_lib):
 
 
 @pytest.mark.parametrize("density_pass", [1, 2], ids=["summation", "shepard"])
+def test_probe_of_a_finished_instance_whose_lists_overflowed(density_pass, native, oracle_lib):
+    """Its lists ask for no rebuild, and a partial build for the other instance keeps them."""
+    a = small_dam(dx=0.05, seed=8, phys=cases.Physics(h_over_dx=2.5))
+    b = cases.periodic_lattice(n_side=12, dx=0.01, seed=3, phys=cases.Physics(g=0.0, density_mode=N.DENSITY_CONTINUITY))
+    b.vel = np.random.default_rng(4).normal(0.0, 2.0, size=b.vel.shape)
+    with Solver(a.n + b.n, max_instances=2, precision=N.PREC_TILED, list_interval=1000, autotune=False) as s:
+        ka, kb = s.add(a, t_end=1e-9), s.add(b)
+        s.step(30)
+        sched = s.list_schedule()
+        assert s.status(ka)["steps"] == 1 and sched["partial_builds"] >= 2 and sched["list_steps"] >= 5, sched
+        for _ in range(30):  # to a step that has just built in part
+            s.step(1)
+            if s.list_schedule()["partial_builds"] > sched["partial_builds"]:
+                break
+        assert s.list_schedule()["partial_builds"] == sched["partial_builds"] + 1
+        st = s.read(ka)
+        pr = s.probe(ka, density_pass=density_pass, lists=True)
+        check(oracle_lib, b, s.read(kb), s.probe(kb, lists=True), N.PREC_TILED)
+    r = oracle_list_check(oracle_lib, a, st, pr, density_pass)
+    np.testing.assert_array_equal(pr["nbr"], r["cnt"])
+    assert r["dens"] < 1e-5 and r["acc"] < 1e-5 and r["div_v"] < 1e-5, r
+
+
+@pytest.mark.parametrize("density_pass", [1, 2], ids=["summation", "shepard"])
 @PRECS
 def test_probe_of_overflowed_lists(prec, density_pass, native, oracle_lib):
     """Particles with more neighbours than a list holds (about 500 at h = 2.5

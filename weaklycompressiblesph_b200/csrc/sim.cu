@@ -1545,6 +1545,7 @@ static int enqueue_probe_lists(SimImpl& S, int density_pass) {
   a.list_reuse = 1;
   a.x0 = S.x0;
   a.alt = a.main;
+  a.inst_keep = nullptr;  // which lists the last build kept is no matter here
   const int n = S.n_host;
   a.zero_pairs = 1;
   k_step_begin<<<1, begin_threads(S), 0, S.s>>>(a);
@@ -1552,7 +1553,9 @@ static int enqueue_probe_lists(SimImpl& S, int density_pass) {
     k_kick_refresh<<<nblk(n), kBlock, 0, S.s>>>(a, 0, 0);
     if (density_pass) {
       if (int rc = launch_density_list(a, n, S.s, h16_lists(S.opt))) return rc;
-      k_density_overflow<<<nblk(n), kBlock, 0, S.s>>>(a);  // no particle has moved since a build that overflowed
+      // no particle of an overflowed list has moved since its build: the next step
+      // builds again, or its instance is finished
+      k_density_overflow<<<nblk(n), kBlock, 0, S.s>>>(a);
       k_eos<<<nblk(n), kBlock, 0, S.s>>>(a);
     }
     const bool h16 = S.opt.precision == WCSPH_PREC_HALF2;
